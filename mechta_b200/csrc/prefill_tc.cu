@@ -1,33 +1,34 @@
-// Prefill attention over the f16 cache on the 5th-generation tensor cores: tcgen05.mma with the S and O
-// accumulators in tensor memory, K/V tiles staged by TMA.
+// Prefill attention over the f16 cache on the 5th-generation tensor cores: tcgen05.mma by CTA pairs, with the S and O
+// accumulators and the queries in tensor memory, K/V tiles staged by TMA.
 //
 // Stands in for q_f16 + attn_fa_mx + attn_fd_combine (W/fa_mx.wgsl:19-115,313-319; M/engine.rs:1215-1226): token T
 // of the block (at pos0 + T) sees first_pos <= key < pos0 + 1 + T; the block's K/V rows were appended before
-// (M/engine.rs:1213-1214). A work item is 16 tokens x the 8 query heads of one KV head = 128 rows (row = head * 16
-// + token, the reference's row order, W/fa_mx.wgsl:4), i.e. one 128-lane TMEM accumulator; every K/V tile feeds all
-// 8 heads.
+// (M/engine.rs:1213-1214).
 //
-// Scheduling. The reference prefills in blocks of 512, 128, 32 and 8 tokens (M/engine.rs:869-885): a 512-token block
-// is 64 items, which as one CTA per item leaves 84 of 148 SMs idle. For launches with fewer items than three
-// quarters of the SMs the grid is therefore one CTA per SM, and the 64-key tiles of all items, laid end to end
-// (longest items first), are cut into equal ranges, one per CTA. A CTA walks its range segment by segment; a
-// segment that covers its whole item writes the output, a part of an item writes its un-normalised partial
-// (reference maximum, sum, O) to scratch memory, and whichever part of the item finishes last merges the parts in
-// index order (the reference splits long prefills over chunks and merges with attn_fd_combine in the same way,
-// M/engine.rs:1219-1225). Measured over a 32,768-token prefix: 128 tokens 0.51 -> 0.41 ms, 512 tokens 0.52 -> 0.40 ms.
-// Larger launches run one CTA per item: with most SMs busy the kernel is bound by the L2 -> SM traffic of the K/V
-// tiles (64 KB per 128 rows and tile, about 8 TB/s), so evening out the waves buys nothing there and the partials
-// cost (1,024 tokens 0.52 -> 0.60 ms, 2,048 tokens 1.06 -> 1.10 ms when split).
+// A work item is 32 tokens x the 8 query heads of one KV head = 256 rows: the M = 256 of a tcgen05.mma.cta_group::2, 128
+// rows in each CTA of a pair (16 tokens a CTA, row = head * 16 + token, the reference's row order, W/fa_mx.wgsl:4). The two
+// CTAs share every K/V tile of 128 keys: each loads one half of it (64 keys of K, 128 of the 256 dims of V) into its own
+// shared memory and the tensor cores of both read both halves. With one CTA per 128 rows the kernel was bound by the L2 ->
+// SM traffic of the tiles (9.1 GB a layer at 2,048 tokens over a 32,768-token prefix, 8.7 TB/s with the products switched
+// off) and by the issue of products with N = 64; a pair needs half the traffic, and its products are 256x128x16 and
+// 256x256x16. Measured, ten layers of 2,048 tokens over 32,768: 12.3 -> 9.7 ms (1,170 TFLOP/s under the power cap; a few layers
+// in a burst run at 1,345). The waits use mbarrier.try_wait at its default scope: with .acquire.cluster, which costs a cache
+// invalidation each time, the same kernel took 1,032 us a layer instead of 843.
 //
-// Roles (192 threads): warp 0 = TMA producer, warp 1 = MMA issuer (one thread) and TMEM owner, warps 2..5 = one
-// softmax thread per row. Per 64-key tile: S = Q K^T (16 MMAs 128x64x16 into one of two S buffers in TMEM);
-// the row's thread reads S, scales, masks, exponentiates against a reference maximum that only moves when the
-// tile maximum exceeds it by more than 8 (the reference's lazy maximum, M/dmx.rs:80 and W/fa_mx.wgsl:120: a
-// matrix accumulator cannot be rescaled per row cheaply), writes P as f16 to shared memory; O += P V (4 MMAs
-// 128x256x16, V used N-major straight from its TMA tile). S of tile j+1 is computed while tile j is in softmax.
-// TMEM: O = columns 0..255, S buffers = 256..319 and 320..383, Q (f16, the A operand of Q K^T) = 384..511, which
-// leaves shared memory to a 3-deep K/V ring; the producer runs ahead across segment borders. Every wait is
-// bounded; TMEM is freed on every path.
+// Scheduling. The grid is one pair of CTAs per two SMs, and the 128-key tiles of all items, laid end to end (longest items
+// first), are cut into equal ranges, one per pair. A pair walks its range segment by segment; a segment that covers its whole
+// item writes the output, a part of an item writes its un-normalised partial (reference maximum, sum, O) to scratch memory,
+// and a second small kernel merges the parts in index order over the whole chip (the reference splits long prefills over
+// chunks and merges with attn_fd_combine in the same way, M/engine.rs:1219-1225). 200 tokens over 9,001: 256 -> 52 us a layer
+// (one CTA per split item used to merge it alone, with uncoalesced loads).
+//
+// Roles (320 threads): warp 0 = TMA producer, warp 1 = MMA issuer (one thread, of the pair's first CTA only) and TMEM owner,
+// warps 2..9 = softmax, two threads per row (64 of a tile's 128 keys each). Per tile: S = Q K^T (16 MMAs, A = Q from tensor
+// memory); the row's threads read S, release it (so that the next tile's S is computed while this one is in softmax), scale,
+// mask, exponentiate against a reference maximum that only moves when the tile exceeds it by more than 8 (the reference's
+// lazy maximum, M/dmx.rs:80 and W/fa_mx.wgsl:120: a matrix accumulator cannot be rescaled per row cheaply), write P as f16 to
+// shared memory; O += P V (8 MMAs, V used N-major straight from its TMA tile).
+// TMEM: O = columns 0..255, S = 256..383, Q (f16) = 384..511. Every wait is bounded; TMEM is freed on every path.
 #include <stdlib.h>
 
 #include <algorithm>
@@ -38,26 +39,34 @@
 namespace mkv {
 using namespace ptx;
 
-constexpr int TC_NST = 3;                              // K/V ring depth
-constexpr uint32_t TC_TILE = 64;                       // keys per tile (= PF_TILE, the tensor map's box)
-constexpr uint32_t TC_KV_STAGE = 65536;                // K 32 KB + V 32 KB
-constexpr uint32_t TC_SUB = 8192;                      // [64 keys][64 dims] f16
-constexpr uint32_t TC_OFF_P = TC_NST * TC_KV_STAGE;    // [128 rows][64 keys] f16
-constexpr uint32_t TC_OFF_BAR = TC_OFF_P + 16384;
-// barriers: kv_full[NST], kv_empty[NST], s_full[2], p_full, pv_done, q_full
-constexpr uint32_t TC_NBAR = 2 * TC_NST + 5;
+constexpr int TC_NST = 3;                              // ring depth, K and V each
+constexpr uint32_t TC_TILE = 128;                      // keys per tile
+constexpr uint32_t TC_BOX = 8192;                      // one TMA box [64 keys][64 dims] f16 (PF_TILE rows)
+constexpr uint32_t TC_HALF = 32768;                    // a CTA's half of a K or V tile
+constexpr uint32_t TC_OFF_V = TC_NST * TC_HALF;
+constexpr uint32_t TC_OFF_P = 2 * TC_NST * TC_HALF;    // [2 key blocks][128 rows][64 keys] f16
+constexpr uint32_t TC_OFF_RED = TC_OFF_P + 32768;      // [2 halves][128 rows] floats
+constexpr uint32_t TC_OFF_BAR = TC_OFF_RED + 1024;
+// barriers: k_full[NST], v_full[NST], k_empty[NST], v_empty[NST], s_full, s_free, p_full, pv_done, q_full
+constexpr uint32_t TC_NBAR = 4 * TC_NST + 5;
 constexpr uint32_t TC_OFF_MISC = TC_OFF_BAR + TC_NBAR * 8; // TcShared
 constexpr uint32_t TC_SMEM = TC_OFF_MISC + 32 + 1024;
 constexpr uint32_t TC_COL_O = 0, TC_COL_S = 256, TC_COL_Q = 384, TC_COLS = 512;
+constexpr int TC_THREADS = 320;
+constexpr int TC_ROW_OUTSIDE = 1 << 30;                // a row coordinate beyond any cache: TMA fills such a box with zeros
 constexpr long long TC_WAIT_LIMIT = 2000000000ll;
-constexpr float TC_LAZY = 8.0f;
-constexpr uint32_t TC_PART = 128 * REC;   // floats of one partial: [128 rows][m, l, O[256]]
-constexpr uint32_t TC_MAX_ITEMS = 512;    // 4,096 tokens / 16 x 2 KV heads
+constexpr float TC_LOG2E = 1.4426950408889634f;
+constexpr float TC_LAZY2 = 8.0f * TC_LOG2E;
+constexpr float TC_C2 = SCALE * TC_LOG2E;              // scores to base-2 exponents
+constexpr uint32_t TC_MIN_LEN = 2;                     // tiles a pair takes at least: a shorter range costs more in partials than it saves
+// One partial of a CTA: O as [64 chunks of 4 dims][128 rows][4] (a warp's rows store and load 512 contiguous bytes), then
+// [128 rows][m, l]
+constexpr size_t TC_PART = 128u * 256u + 128u * 2u;
+static_assert(TC_SMEM <= 232448, "shared memory of prefill_f16_tc_kernel");
 
 struct TcShared {
     uint32_t tmem_base;
     volatile uint32_t abort;
-    uint32_t ticket;
 };
 
 // Bounded wait shared by all roles: returns false (and raises the CTA's abort flag) when it runs out or when
@@ -69,77 +78,59 @@ __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, TcShared 
     atomicOr(status, DEV_ERR_WAIT_TIMEOUT);
     return false;
 }
-// named barrier 1: the 128 softmax threads
-__device__ __forceinline__ void tc_bar_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
-// The work of one launch and this CTA's share of it. Items are numbered longest first: item i = (token group
-// ngroups - 1 - i / 2, KV head i % 2); its tiles are the 64-key tiles from first_pos / 64 up to the last key its
-// last token sees. Every thread computes the same plan (a few hundred integer operations against a kernel of about
-// a millisecond).
-struct PfWork {
-    uint32_t first_pos, pos0, ntok, ngroups, nitems, t0;
-    uint32_t lo, hi, len; // this CTA's range [lo, hi) of the tiles laid end to end, the length of every CTA's range
-    bool split;
-    __device__ __forceinline__ uint32_t tiles_of(uint32_t item) const {
+// The work of one launch. Items are numbered longest first: item i = (group of 32 tokens ngroups - 1 - i / 2, KV head i % 2);
+// its tiles are the 128-key tiles from first_pos / 128 up to the last key its last token sees. Pair p takes the tiles
+// [p * len, (p + 1) * len) of all items laid end to end.
+struct PfPlan {
+    uint32_t first_pos, pos0, ntok;
+    uint32_t ngroups, nitems, t0;
+    uint32_t total, len;
+    __host__ __device__ uint32_t tiles_of(uint32_t item) const {
         const uint32_t grp = ngroups - 1u - (item >> 1);
-        const uint32_t last_tok = min(grp * 16u + 15u, ntok - 1u);
-        return (pos0 + 1u + last_tok + TC_TILE - 1u) / TC_TILE - t0;
+        const uint32_t last = grp * 32u + 31u < ntok - 1u ? grp * 32u + 31u : ntok - 1u;
+        return (pos0 + last + TC_TILE) / TC_TILE - t0;
     }
 };
 struct PfSegment {
     uint32_t item, a, b;     // tiles [a, b) of the item
     uint32_t piece, npieces; // which part of the item this is, of how many
-    uint32_t cta0;           // the CTA that holds the item's first part
 };
-__device__ __forceinline__ PfWork pf_work(uint32_t first_pos, uint32_t pos0, uint32_t ntok, bool split) {
-    PfWork w;
-    w.first_pos = first_pos; w.pos0 = pos0; w.ntok = ntok;
-    w.ngroups = (ntok + 15u) / 16u;
-    w.nitems = 2u * w.ngroups;
-    w.t0 = first_pos / TC_TILE;
-    w.split = split;
-    if (w.split) {
-        uint32_t total = 0;
-        for (uint32_t i = 0; i < w.nitems; i += 2u) total += 2u * w.tiles_of(i);
-        w.len = (total + gridDim.x - 1u) / gridDim.x;
-        w.lo = blockIdx.x * w.len;
-        w.hi = min(w.lo + w.len, total);
-    } else {
-        w.len = w.lo = w.hi = 0;
+// Walks the segments of one pair.
+struct PfWalk {
+    const PfPlan &p;
+    uint32_t pair, lo, hi, item, base;
+    __device__ __forceinline__ PfWalk(const PfPlan &plan, uint32_t pair_) : p(plan), pair(pair_), item(0), base(0) {
+        lo = min(pair * p.len, p.total);
+        hi = min(lo + p.len, p.total);
     }
-    return w;
-}
-// Calls f(segment) for this CTA's segments in order; f returns false to stop. Returns false if f did.
-template <typename F>
-__device__ __forceinline__ bool pf_segments(const PfWork &w, F &&f) {
-    if (!w.split) { // one whole item per CTA
-        PfSegment sg = {blockIdx.x, 0u, w.tiles_of(blockIdx.x), 0u, 1u, blockIdx.x};
-        return f(sg);
-    }
-    uint32_t base = 0;
-    for (uint32_t i = 0; i < w.nitems && base < w.hi; i++) {
-        const uint32_t n = w.tiles_of(i);
-        const uint32_t lo = max(base, w.lo), hi = min(base + n, w.hi);
-        if (hi > lo) {
-            const uint32_t c0 = base / w.len;
-            PfSegment sg = {i, lo - base, hi - base, blockIdx.x - c0, (base + n - 1u) / w.len - c0 + 1u, c0};
-            if (!f(sg)) return false;
+    __device__ __forceinline__ bool next(PfSegment &s) {
+        while (item < p.nitems && base < hi) {
+            const uint32_t n = p.tiles_of(item), a = max(base, lo), b = min(base + n, hi);
+            if (b > a) {
+                const uint32_t c0 = base / p.len;
+                s = {item, a - base, b - base, pair - c0, (base + n - 1u) / p.len - c0 + 1u};
+            }
+            const bool found = b > a;
+            base += n;
+            item++;
+            if (found) return true;
         }
-        base += n;
+        return false;
     }
-    return true;
+};
+// Where a pair's CTA keeps the partial of a part: a pair has at most one segment that continues an item begun by the pair
+// before it (slot 0) and at most one that begins an item it does not finish (slot 1).
+__host__ __device__ inline size_t pf_slot(uint32_t pair, uint32_t piece, uint32_t cta) {
+    return ((size_t)pair * 2u + (piece == 0u ? 1u : 0u)) * 2u + cta;
 }
-// Where part `piece` of an item whose first part lies in CTA cta0 keeps its partial: a CTA has at most one segment
-// that continues an item begun by the CTA before it (slot 0) and at most one that begins an item it does not finish (slot 1).
-__device__ __forceinline__ size_t pf_slot(uint32_t cta0, uint32_t piece) { return 2u * (size_t)(cta0 + piece) + (piece == 0u ? 1u : 0u); }
 
 // QF16: the queries come as f16 [ntok][16][256] (the output of the reference's q_f16 pass) instead of f32.
 template <bool QF16>
-__global__ void __launch_bounds__(192, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
 prefill_f16_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
-                      const void *__restrict__ q, float *__restrict__ out, uint32_t first_pos, uint32_t pos0, uint32_t ntok,
-                      uint32_t row0, float *__restrict__ scratch, uint32_t *__restrict__ counters, uint32_t split,
-                      uint32_t *__restrict__ status, uint32_t phase_arg) {
+                      const void *__restrict__ q, float *__restrict__ out, const __grid_constant__ PfPlan plan, uint32_t row0,
+                      float *__restrict__ scratch, uint32_t *__restrict__ status, uint32_t phase_arg) {
     // phase (builds with -DMKV_MEASURE only): 0 = everything, 1 = tile loads only, 2 = loads and MMAs without the softmax math
 #ifdef MKV_MEASURE
     const uint32_t phase = phase_arg;
@@ -148,250 +139,297 @@ prefill_f16_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
     (void)phase_arg;
 #endif
     extern __shared__ uint8_t smem_raw[];
-    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u; // the same in both CTAs
     uint8_t *smem = smem_raw + (smem_base - smem_u32(smem_raw));
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+    const uint32_t cta = cluster_ctarank(), pair = blockIdx.x >> 1;
     const uint32_t bar0 = smem_base + TC_OFF_BAR;
-    const uint32_t bar_kv_full = bar0, bar_kv_empty = bar0 + 8u * TC_NST, bar_s_full = bar0 + 16u * TC_NST;
-    const uint32_t bar_p_full = bar_s_full + 16u, bar_pv_done = bar_p_full + 8u, bar_q_full = bar_pv_done + 8u;
+    const uint32_t bar_k_full = bar0, bar_v_full = bar0 + 8u * TC_NST, bar_k_empty = bar0 + 16u * TC_NST, bar_v_empty = bar0 + 24u * TC_NST;
+    const uint32_t bar_s_full = bar0 + 32u * TC_NST, bar_s_free = bar_s_full + 8u, bar_p_full = bar_s_free + 8u;
+    const uint32_t bar_pv_done = bar_p_full + 8u, bar_q_full = bar_pv_done + 8u;
     TcShared *sh = reinterpret_cast<TcShared *>(smem + TC_OFF_MISC);
-    const PfWork work = pf_work(first_pos, pos0, ntok, split != 0u);
+    pdl_launch_dependents();
 
     if (tid == 0) {
-        for (int s = 0; s < TC_NST; s++) {
-            mbar_init(bar_kv_full + 8u * s, 1);
-            mbar_init(bar_kv_empty + 8u * s, 1);
-        }
+        for (int s = 0; s < 4 * TC_NST; s++) mbar_init(bar0 + 8u * s, 1);
         mbar_init(bar_s_full, 1);
-        mbar_init(bar_s_full + 8u, 1);
-        mbar_init(bar_p_full, 128);
+        mbar_init(bar_s_free, 16); // one arrival per softmax warp of the pair (counted in the first CTA only)
+        mbar_init(bar_p_full, 16);
         mbar_init(bar_pv_done, 1);
-        mbar_init(bar_q_full, 128);
+        mbar_init(bar_q_full, 16);
         sh->abort = 0;
         fence_barrier_init();
         fence_proxy_async();
     }
-    if (warp == 1) tmem_alloc(smem_base + TC_OFF_MISC, TC_COLS); // writes sh->tmem_base
-
+    if (warp == 1) tmem_alloc2(smem_base + TC_OFF_MISC, TC_COLS); // writes sh->tmem_base
     tc_fence_before();
-    __syncthreads();
+    cluster_sync(); // barriers and tensor memory of both CTAs are there
     tc_fence_after();
     const uint32_t tmem = sh->tmem_base;
+    pdl_wait(); // nothing global is touched before the kernel in front has finished
 
-    // Every role walks the same segments; g counts the tiles this CTA has dealt with so far, across segments: ring
-    // stage g % NST, S buffer g & 1, and the parities of the barriers follow from it.
+    // Every role walks the same segments; g counts the tiles this pair has dealt with so far, across segments: ring
+    // stage g % NST and the parities of the barriers follow from it.
     if (warp == 0) {
         // ---------------- TMA producer: runs ahead of the other roles, also across segment borders ----------------
         if (lane == 0) {
             uint32_t g = 0;
-            pf_segments(work, [&](const PfSegment &sg) {
+            PfWalk walk(plan, pair);
+            PfSegment sg;
+            bool ok = true;
+            while (ok && walk.next(sg)) {
                 const int x = (int)((sg.item & 1u) * 256u);
+                const uint32_t end = plan.pos0 + plan.ntok; // no key at or past this one is seen by anybody
                 for (uint32_t j = sg.a; j < sg.b; j++, g++) {
-                    const uint32_t s = g % TC_NST;
-                    if (g >= (uint32_t)TC_NST && !tc_wait(bar_kv_empty + 8u * s, ((g / TC_NST) - 1u) & 1u, sh, status)) return false;
-                    const uint32_t dst = smem_base + s * TC_KV_STAGE, bar = bar_kv_full + 8u * s;
-                    const int y = (int)((work.t0 + j) * TC_TILE - row0);
-                    mbar_expect_tx(bar, TC_KV_STAGE);
+                    const uint32_t s = g % TC_NST, key0 = (plan.t0 + j) * TC_TILE;
+                    const int y[2] = {(int)(key0 - row0), key0 + 64u < end ? (int)(key0 + 64u - row0) : TC_ROW_OUTSIDE};
+                    const uint32_t par = ((g / TC_NST) - 1u) & 1u;
+                    if (g >= (uint32_t)TC_NST && !(ok = tc_wait(bar_k_empty + 8u * s, par, sh, status))) break;
+                    // both CTAs' halves are counted on the first CTA's barrier: its MMA thread is the one that waits
+                    uint32_t dst = smem_base + s * TC_HALF, bar = cluster_map(bar_k_full + 8u * s, 0);
+                    if (cta == 0) mbar_expect_tx(bar_k_full + 8u * s, 2u * TC_HALF);
 #pragma unroll
-                    for (int sb = 0; sb < 4; sb++) tma_load_2d(dst + sb * TC_SUB, &kmap, x + 64 * sb, y, bar);
+                    for (int db = 0; db < 4; db++) tma_load_2d_pair(dst + db * TC_BOX, &kmap, x + 64 * db, y[cta], bar);
+                    if (g >= (uint32_t)TC_NST && !(ok = tc_wait(bar_v_empty + 8u * s, par, sh, status))) break;
+                    dst = smem_base + TC_OFF_V + s * TC_HALF;
+                    bar = cluster_map(bar_v_full + 8u * s, 0);
+                    if (cta == 0) mbar_expect_tx(bar_v_full + 8u * s, 2u * TC_HALF);
 #pragma unroll
-                    for (int sb = 0; sb < 4; sb++) tma_load_2d(dst + 4 * TC_SUB + sb * TC_SUB, &vmap, x + 64 * sb, y, bar);
+                    for (int db = 0; db < 2; db++)
+#pragma unroll
+                        for (int kb = 0; kb < 2; kb++)
+                            tma_load_2d_pair(dst + (2 * db + kb) * TC_BOX, &vmap, x + 128 * (int)cta + 64 * db, y[kb], bar);
                 }
-                return true;
-            });
+            }
+            // the last releases must have arrived here before this CTA may leave: they come from the other CTA's commits
+            for (uint32_t i = g > (uint32_t)TC_NST ? g - TC_NST : 0u; ok && i < g; i++)
+                ok = tc_wait(bar_k_empty + 8u * (i % TC_NST), (i / TC_NST) & 1u, sh, status) &&
+                     tc_wait(bar_v_empty + 8u * (i % TC_NST), (i / TC_NST) & 1u, sh, status);
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            constexpr uint32_t IDESC_QK = tc_idesc_f16(128, 64, false);
-            constexpr uint32_t IDESC_PV = tc_idesc_f16(128, 256, true);
+        if (lane == 0 && cta == 0) {
+            constexpr uint32_t IDESC_QK = tc_idesc_f16(256, 128, false);
+            constexpr uint32_t IDESC_PV = tc_idesc_f16(256, 256, true);
             uint32_t g = 0, nseg = 0;
-            auto qk = [&](uint32_t gg) -> bool { // S[gg & 1] = Q K^T for the tile in ring stage gg % NST
+            auto qk = [&](uint32_t gg) -> bool { // S = Q K^T for tile gg
                 const uint32_t s = gg % TC_NST;
-                if (!tc_wait(bar_kv_full + 8u * s, (gg / TC_NST) & 1u, sh, status)) return false;
+                if (gg > 0u && !tc_wait(bar_s_free, (gg - 1u) & 1u, sh, status)) return false;
+                if (!tc_wait(bar_k_full + 8u * s, (gg / TC_NST) & 1u, sh, status)) return false;
                 tc_fence_after();
-                const uint32_t kb = smem_base + s * TC_KV_STAGE;
-                const uint32_t d = tmem + TC_COL_S + 64u * (gg & 1u);
+                const uint32_t kb = smem_base + s * TC_HALF;
 #pragma unroll
-                for (uint32_t ks = 0; ks < 16u; ks++) { // 16 dims per MMA; 4 per 64-dim sub-box
-                    const uint64_t b = tc_desc_sw128(kb + (ks >> 2) * TC_SUB + (ks & 3u) * 32u, 16, 1024);
-                    if (phase != 1u) tc_mma_f16_ta(d, tmem + TC_COL_Q + 8u * ks, b, IDESC_QK, ks > 0 ? 1u : 0u);
+                for (uint32_t ks = 0; ks < 16u; ks++) { // 16 dims per MMA; 4 per 64-dim box
+                    const uint64_t b = tc_desc_sw128(kb + (ks >> 2) * TC_BOX + (ks & 3u) * 32u, 16, 1024);
+                    if (phase != 1u) tc_mma2_f16_ta(tmem + TC_COL_S, tmem + TC_COL_Q + 8u * ks, b, IDESC_QK, ks > 0 ? 1u : 0u);
                 }
-                tc_commit(bar_s_full + 8u * (gg & 1u));
+                tc_commit2(bar_k_empty + 8u * s);
+                tc_commit2(bar_s_full);
                 return true;
             };
-            pf_segments(work, [&](const PfSegment &sg) {
-                // the segment's Q is in tensor memory (the softmax threads put it there once the MMAs of the segment
-                // before it had all completed)
-                if (!tc_wait(bar_q_full, nseg & 1u, sh, status)) return false;
+            PfWalk walk(plan, pair);
+            PfSegment sg;
+            bool ok = true;
+            while (ok && walk.next(sg)) {
+                // the segment's Q is in tensor memory (the softmax threads put it there once the scores of the segment
+                // before it were all there)
+                if (!(ok = tc_wait(bar_q_full, nseg & 1u, sh, status))) break;
                 tc_fence_after();
                 nseg++;
                 const uint32_t n = sg.b - sg.a;
-                if (!qk(g)) return false;
+                if (!(ok = qk(g))) break;
                 for (uint32_t j = 0; j < n; j++, g++) {
-                    if (j + 1u < n && !qk(g + 1u)) return false; // the next tile's scores while this one is in softmax
-                    if (!tc_wait(bar_p_full, g & 1u, sh, status)) return false;
+                    if (j + 1u < n && !(ok = qk(g + 1u))) break; // the next tile's scores while this one is in softmax
+                    const uint32_t s = g % TC_NST;
+                    if (!(ok = tc_wait(bar_v_full + 8u * s, (g / TC_NST) & 1u, sh, status))) break;
+                    if (!(ok = tc_wait(bar_p_full, g & 1u, sh, status))) break;
                     tc_fence_after();
-                    const uint32_t vb = smem_base + (g % TC_NST) * TC_KV_STAGE + 4 * TC_SUB, pb = smem_base + TC_OFF_P;
+                    const uint32_t vb = smem_base + TC_OFF_V + s * TC_HALF, pb = smem_base + TC_OFF_P;
 #pragma unroll
-                    for (uint32_t ks = 0; ks < 4u; ks++) { // 16 keys per MMA
-                        const uint64_t a = tc_desc_sw128(pb + ks * 32u, 16, 1024);
-                        // V tile [64 keys][64 dims] x 4 sub-boxes, N-major: next 64 dims 8192 bytes on, next 8 keys 1024
-                        const uint64_t b = tc_desc_sw128(vb + ks * 2048u, TC_SUB, 1024);
-                        if (phase != 1u) tc_mma_f16(tmem + TC_COL_O, a, b, IDESC_PV, (j > 0 || ks > 0) ? 1u : 0u);
+                    for (uint32_t ks = 0; ks < 8u; ks++) { // 16 keys per MMA
+                        const uint64_t a = tc_desc_sw128(pb + (ks >> 2) * 16384u + (ks & 3u) * 32u, 16, 1024);
+                        // V half [2 blocks of 64 dims][128 keys], N-major: the next 64 dims 16 KB on, the next 8 keys 1024 bytes
+                        const uint64_t b = tc_desc_sw128(vb + ks * 2048u, 2u * TC_BOX, 1024);
+                        if (phase != 1u) tc_mma2_f16(tmem + TC_COL_O, a, b, IDESC_PV, (j > 0 || ks > 0) ? 1u : 0u);
                     }
-                    tc_commit(bar_kv_empty + 8u * (g % TC_NST)); // K and V of the stage are free
-                    tc_commit(bar_pv_done);                      // O holds the segment's tiles so far; P may be overwritten
+                    tc_commit2(bar_v_empty + 8u * s);
+                    tc_commit2(bar_pv_done); // O holds the segment's tiles so far; P may be overwritten
                 }
-                return true;
-            });
+            }
         }
     } else {
-        // ---------------- softmax: one thread per row (TMEM lane) ----------------
-        const uint32_t row = 32u * (warp & 3u) + lane; // the TMEM lanes this warp may access
-        const uint32_t lane_addr = (32u * (warp & 3u)) << 16;
-        uint32_t g = 0;
-        pf_segments(work, [&](const PfSegment &sg) {
-            const uint32_t grp = work.ngroups - 1u - (sg.item >> 1), kvh = sg.item & 1u;
-            const uint32_t tok0 = grp * 16u;
-            const uint32_t tok = tok0 + (row & 15u), head = 8u * kvh + (row >> 4);
-            const uint32_t vis = pos0 + 1u + tok;              // the row's token sees keys < vis
-            const uint32_t full_below = pos0 + 1u + tok0;      // keys below this are visible to every row
-            bool ok = true;
-            // Q of the item goes to tensor memory as the A operand of S = Q K^T (q_f16 of the reference,
-            // W/fa_mx.wgsl:313-319): the thread that owns a row converts it to f16 and stores it in its lane, two
-            // values per 32-bit column. Q in TMEM instead of shared memory leaves room for a third K/V stage. The MMAs
-            // of the segment before this one have completed: its epilogue waited for them.
-            {
-                const size_t qoff = (size_t)min(tok, ntok - 1u) * 4096u + (size_t)head * 256u;
-#pragma unroll 1
-                for (uint32_t c0 = 0; c0 < 4u; c0++) { // 64 dims = 32 columns per store
-                    uint32_t w[32];
-                    if constexpr (QF16) { // already f16: eight 16-byte loads per 64 dims
-                        const uint4 *src = reinterpret_cast<const uint4 *>(static_cast<const __half *>(q) + qoff + c0 * 64u);
+        // ---------------- softmax: two threads per row (TMEM lane), 64 keys of a tile and 128 dims of O each ----------------
+        const uint32_t q4 = warp & 3u, half = (warp - 2u) >> 2;
+        const uint32_t row = 32u * q4 + lane; // the TMEM lanes this warp may access
+        const uint32_t lane_addr = (32u * q4) << 16;
+        const uint32_t r_s_free = cluster_map(bar_s_free, 0), r_p_full = cluster_map(bar_p_full, 0), r_q_full = cluster_map(bar_q_full, 0);
+        float *red = reinterpret_cast<float *>(smem + TC_OFF_RED);
+        auto arrive = [&](uint32_t bar) { // one arrival per warp, after all its lanes
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(bar);
+        };
+        // Q of an item goes to tensor memory as the A operand of S = Q K^T (q_f16 of the reference, W/fa_mx.wgsl:313-319):
+        // a row's thread converts 128 of its 256 values to f16 and stores them in its lane, two per 32-bit column.
+        auto load_q = [&](const PfSegment &sg) {
+            const uint32_t tok = (plan.ngroups - 1u - (sg.item >> 1)) * 32u + 16u * cta + (row & 15u), head = 8u * (sg.item & 1u) + (row >> 4);
+            const size_t qoff = (size_t)min(tok, plan.ntok - 1u) * 4096u + (size_t)head * 256u + 128u * half;
 #pragma unroll
-                        for (int i = 0; i < 8; i++) {
-                            const uint4 a = src[i];
-                            w[4 * i] = a.x; w[4 * i + 1] = a.y; w[4 * i + 2] = a.z; w[4 * i + 3] = a.w;
-                        }
-                    } else {
-                        const float *src = static_cast<const float *>(q) + qoff + c0 * 64u;
+            for (uint32_t c0 = 0; c0 < 2u; c0++) { // 64 dims = 32 columns per store
+                uint32_t w[32];
+                if constexpr (QF16) { // already f16: eight 16-byte loads per 64 dims
+                    const uint4 *src = reinterpret_cast<const uint4 *>(static_cast<const __half *>(q) + qoff + c0 * 64u);
 #pragma unroll
-                        for (int i = 0; i < 16; i++) {
-                            const float4 a = *reinterpret_cast<const float4 *>(src + 4 * i);
-                            const __half2 h0 = __floats2half2_rn(a.x, a.y), h1 = __floats2half2_rn(a.z, a.w);
-                            w[2 * i] = *reinterpret_cast<const uint32_t *>(&h0);
-                            w[2 * i + 1] = *reinterpret_cast<const uint32_t *>(&h1);
-                        }
+                    for (int i = 0; i < 8; i++) {
+                        const uint4 a = src[i];
+                        w[4 * i] = a.x; w[4 * i + 1] = a.y; w[4 * i + 2] = a.z; w[4 * i + 3] = a.w;
                     }
-                    if (tok >= ntok) {
+                } else {
+                    const float *src = static_cast<const float *>(q) + qoff + c0 * 64u;
 #pragma unroll
-                        for (int i = 0; i < 32; i++) w[i] = 0u;
+                    for (int i = 0; i < 16; i++) {
+                        const float4 a = *reinterpret_cast<const float4 *>(src + 4 * i);
+                        const __half2 h0 = __floats2half2_rn(a.x, a.y), h1 = __floats2half2_rn(a.z, a.w);
+                        w[2 * i] = *reinterpret_cast<const uint32_t *>(&h0);
+                        w[2 * i + 1] = *reinterpret_cast<const uint32_t *>(&h1);
                     }
-                    tmem_st32(tmem + lane_addr + TC_COL_Q + 32u * c0, w);
                 }
-                tmem_wait_st();
-                tc_fence_before();
-                mbar_arrive(bar_q_full);
+                if (tok >= plan.ntok) {
+#pragma unroll
+                    for (int i = 0; i < 32; i++) w[i] = 0u;
+                }
+                tmem_st32(tmem + lane_addr + TC_COL_Q + 64u * half + 32u * c0, w);
             }
-            float m_ref = NEG_BIG, l_run = 0.0f;
+            tmem_wait_st();
+            tc_fence_before();
+            arrive(r_q_full);
+        };
+        uint32_t g = 0;
+        PfWalk walk(plan, pair);
+        PfSegment sg, nx;
+        bool more = walk.next(sg), ok = true;
+        if (more) load_q(sg);
+        while (more) {
+            const uint32_t tok0 = (plan.ngroups - 1u - (sg.item >> 1)) * 32u + 16u * cta, kvh = sg.item & 1u;
+            const uint32_t tok = tok0 + (row & 15u), head = 8u * kvh + (row >> 4);
+            const uint32_t vis = plan.pos0 + 1u + tok;         // the row's token sees keys < vis
+            const uint32_t full_below = plan.pos0 + 1u + tok0; // keys below this are visible to every row of the CTA
+            float m_ref = NEG_BIG, l_run = 0.0f; // l_run: this thread's 64 keys of every tile only
             const uint32_t n = sg.b - sg.a;
             for (uint32_t j = 0; j < n; j++, g++) {
-                // the warp takes every wait's outcome together: the TMEM loads below are warp-collective
-                if (!(ok = __all_sync(0xffffffffu, tc_wait(bar_s_full + 8u * (g & 1u), (g >> 1) & 1u, sh, status)))) break;
+                // The warp takes every wait's outcome together: the TMEM loads below are warp-collective. A wait that ran out
+                // goes into the next vote, so that the two warps of these rows leave together.
+                ok = __all_sync(0xffffffffu, tc_wait(bar_s_full, g & 1u, sh, status)) && ok;
                 tc_fence_after();
                 if (phase != 0u) { // measurement: no softmax math, P left as it is
-                    if (j > 0 && !(ok = __all_sync(0xffffffffu, tc_wait(bar_pv_done, (g - 1u) & 1u, sh, status)))) break;
                     tc_fence_before();
-                    mbar_arrive(bar_p_full);
+                    arrive(r_s_free);
+                    if (j > 0) ok = __all_sync(0xffffffffu, tc_wait(bar_pv_done, (g - 1u) & 1u, sh, status)) && ok;
+                    if (!ok) break; // (no vote in this mode before the segment's end)
+                    arrive(r_p_full);
                     continue;
                 }
                 uint32_t sr[2][32];
-                tmem_ld32(tmem + lane_addr + TC_COL_S + 64u * (g & 1u), sr[0]);
-                tmem_ld32(tmem + lane_addr + TC_COL_S + 64u * (g & 1u) + 32u, sr[1]);
+                tmem_ld32(tmem + lane_addr + TC_COL_S + 64u * half, sr[0]);
+                tmem_ld32(tmem + lane_addr + TC_COL_S + 64u * half + 32u, sr[1]);
                 tmem_wait_ld();
-                const uint32_t key_base = (work.t0 + sg.a + j) * TC_TILE;
-                const bool need_mask = key_base + TC_TILE > full_below || key_base < first_pos;
+                tc_fence_before();
+                arrive(r_s_free); // the next tile's scores may be computed
+                const uint32_t key_base = (plan.t0 + sg.a + j) * TC_TILE + 64u * half;
                 // work in base-2 exponents: exp(s / 16 - m) = 2^(s * C - m2), C = log2(e) / 16, one FFMA + one ex2 per score
-                constexpr float C2 = SCALE * 1.4426950408889634f;
-                float mt = NEG_BIG;
-                if (need_mask) { // tiles that touch the causal diagonal or the window start: scale, then mask (W/fa_mx.wgsl:62)
+                float mt[4] = {NEG_BIG, NEG_BIG, NEG_BIG, NEG_BIG};
+                if (key_base + 64u > full_below || key_base < plan.first_pos) { // the causal diagonal or the window start (W/fa_mx.wgsl:62)
 #pragma unroll
                     for (int h = 0; h < 2; h++)
 #pragma unroll
                         for (int c = 0; c < 32; c++) {
                             const uint32_t key = key_base + 32u * h + c;
-                            const float v = (key >= first_pos && key < vis) ? __uint_as_float(sr[h][c]) : NEG_BIG;
+                            const float v = (key >= plan.first_pos && key < vis) ? __uint_as_float(sr[h][c]) : NEG_BIG;
                             sr[h][c] = __float_as_uint(v);
-                            mt = fmaxf(mt, v);
+                            mt[c & 3] = fmaxf(mt[c & 3], v);
                         }
                 } else {
 #pragma unroll
                     for (int h = 0; h < 2; h++)
 #pragma unroll
-                        for (int c = 0; c < 32; c++) mt = fmaxf(mt, __uint_as_float(sr[h][c]));
+                        for (int c = 0; c < 32; c++) mt[c & 3] = fmaxf(mt[c & 3], __uint_as_float(sr[h][c]));
                 }
-                mt = mt > NEG_TEST ? mt * C2 : NEG_BIG; // the tile maximum as a base-2 exponent
-                // lazy reference maximum: move it only for the first valid tile or when the tile exceeds it by more than 8
-                // (in natural units, as the reference; 8 * log2(e) here)
+                float mx = fmaxf(fmaxf(mt[0], mt[1]), fmaxf(mt[2], mt[3]));
+                mx = mx > NEG_TEST ? mx * TC_C2 : NEG_BIG; // this half row's tile maximum as a base-2 exponent
+                // Lazy reference maximum: it moves only for the first valid tile or when the tile exceeds it by more than 8 (in
+                // natural units, as the reference). The two warps that share these 32 rows vote; only then they exchange maxima.
                 float cf = 1.0f;
-                if (mt > NEG_TEST && (m_ref < NEG_TEST || mt > m_ref + TC_LAZY * 1.4426950408889634f)) {
-                    const float m_new = fmaxf(m_ref, mt);
-                    cf = m_ref > NEG_TEST ? exp2f(m_ref - m_new) : 1.0f;
-                    m_ref = m_new;
+                if (pair_bar_or(1u + q4, !ok || (mx > NEG_TEST && (m_ref < NEG_TEST || mx > m_ref + TC_LAZY2)))) {
+                    red[128u * half + row] = mx;
+                    if (pair_bar_or(1u + q4, !ok)) {
+                        ok = false;
+                        break;
+                    }
+                    mx = fmaxf(mx, red[128u * (half ^ 1u) + row]);
+                    if (mx > NEG_TEST && (m_ref < NEG_TEST || mx > m_ref + TC_LAZY2)) {
+                        const float m_new = fmaxf(m_ref, mx);
+                        cf = m_ref > NEG_TEST ? exp2f(m_ref - m_new) : 1.0f;
+                        m_ref = m_new;
+                    }
                 }
                 const float neg_m = m_ref > NEG_TEST ? -m_ref : 0.0f; // masked scores stay at -3e38 * C: 2^that = 0
-                float sum = 0.0f;
+                float sum[2] = {0.0f, 0.0f};
                 uint32_t ph[32]; // 64 weights as f16 pairs
 #pragma unroll
                 for (int h = 0; h < 2; h++)
 #pragma unroll
                     for (int c = 0; c < 32; c += 2) {
                         float w0, w1;
-                        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(w0) : "f"(fmaf(__uint_as_float(sr[h][c]), C2, neg_m)));
-                        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(w1) : "f"(fmaf(__uint_as_float(sr[h][c + 1]), C2, neg_m)));
-                        sum += w0 + w1;
+                        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(w0) : "f"(fmaf(__uint_as_float(sr[h][c]), TC_C2, neg_m)));
+                        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(w1) : "f"(fmaf(__uint_as_float(sr[h][c + 1]), TC_C2, neg_m)));
+                        sum[0] += w0;
+                        sum[1] += w1;
                         const __half2 hp = __floats2half2_rn(w0, w1);
                         ph[16 * h + (c >> 1)] = *reinterpret_cast<const uint32_t *>(&hp);
                     }
-                l_run = l_run * cf + sum;
+                l_run = l_run * cf + (sum[0] + sum[1]);
                 // P and O belong to the MMAs of the tile before until those have completed
-                if (j > 0 && !(ok = __all_sync(0xffffffffu, tc_wait(bar_pv_done, (g - 1u) & 1u, sh, status)))) break;
+                if (j > 0) ok = __all_sync(0xffffffffu, tc_wait(bar_pv_done, (g - 1u) & 1u, sh, status));
                 tc_fence_after();
-                if (j > 0 && __any_sync(0xffffffffu, cf != 1.0f)) { // rescale this warp's rows of O (rare)
+                if (j > 0 && __any_sync(0xffffffffu, cf != 1.0f)) { // rescale this warp's rows and dims of O (rare)
 #pragma unroll 1
-                    for (uint32_t c0 = 0; c0 < 256u; c0 += 32u) {
+                    for (uint32_t c0 = 0; c0 < 128u; c0 += 32u) {
                         uint32_t orow[32];
-                        tmem_ld32(tmem + lane_addr + TC_COL_O + c0, orow);
+                        tmem_ld32(tmem + lane_addr + TC_COL_O + 128u * half + c0, orow);
                         tmem_wait_ld();
 #pragma unroll
                         for (int c = 0; c < 32; c++) orow[c] = __float_as_uint(__uint_as_float(orow[c]) * cf);
-                        tmem_st32(tmem + lane_addr + TC_COL_O + c0, orow);
+                        tmem_st32(tmem + lane_addr + TC_COL_O + 128u * half + c0, orow);
                     }
                     tmem_wait_st();
                 }
-                uint8_t *prow = smem + TC_OFF_P;
+                uint8_t *prow = smem + TC_OFF_P + 16384u * half;
 #pragma unroll
                 for (uint32_t c = 0; c < 8u; c++) // 8 chunks of 8 keys
                     *reinterpret_cast<uint4 *>(prow + swz128(row, c)) = make_uint4(ph[4 * c], ph[4 * c + 1], ph[4 * c + 2], ph[4 * c + 3]);
                 fence_proxy_async();
                 tc_fence_before();
-                mbar_arrive(bar_p_full);
+                arrive(r_p_full);
             }
+            // All scores of the segment are there, so its Q may be replaced: the next segment's first scores are computed while
+            // this one's last products and its epilogue run.
+            more = ok && walk.next(nx);
+            if (more) load_q(nx);
             // ---------------- end of the segment: all its MMAs have completed ----------------
-            if (ok && n > 0) ok = __all_sync(0xffffffffu, tc_wait(bar_pv_done, (g - 1u) & 1u, sh, status));
+            ok = ok && __all_sync(0xffffffffu, tc_wait(bar_pv_done, (g - 1u) & 1u, sh, status));
             tc_fence_after();
-            if (!ok) return false;
+            red[128u * half + row] = l_run;
+            if (pair_bar_or(1u + q4, !ok)) break;
+            const float l_all = red[row] + red[128u + row];
             if (sg.npieces == 1u) {
                 // the whole item: out[tok][head][:] = O / l
-                const float inv = 1.0f / l_run;
-                float *dst = out + (size_t)tok * 4096u + (size_t)head * 256u;
+                const float inv = 1.0f / l_all;
+                float *dst = out + (size_t)tok * 4096u + (size_t)head * 256u + 128u * half;
 #pragma unroll 1
-                for (uint32_t c0 = 0; c0 < 256u; c0 += 32u) {
+                for (uint32_t c0 = 0; c0 < 128u; c0 += 32u) {
                     uint32_t orow[32];
-                    tmem_ld32(tmem + lane_addr + TC_COL_O + c0, orow);
+                    tmem_ld32(tmem + lane_addr + TC_COL_O + 128u * half + c0, orow);
                     tmem_wait_ld();
-                    if (tok < ntok) {
+                    if (tok < plan.ntok) {
 #pragma unroll
                         for (int c = 0; c < 32; c += 4)
                             *reinterpret_cast<float4 *>(dst + c0 + c) =
@@ -400,79 +438,94 @@ prefill_f16_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
                     }
                 }
             } else {
-                // a part of an item: its partial goes to scratch memory; the part that arrives last merges all of them
-                float *ps = scratch + pf_slot(sg.cta0, sg.piece) * TC_PART + (size_t)row * REC;
-                *reinterpret_cast<float2 *>(ps) = make_float2(m_ref, l_run);
+                // a part of an item: its partial goes to scratch memory for the merge kernel
+                float *ps = scratch + pf_slot(pair, sg.piece, cta) * TC_PART;
+                if (half == 0u) *reinterpret_cast<float2 *>(ps + 128u * 256u + 2u * row) = make_float2(m_ref, l_all);
 #pragma unroll 1
-                for (uint32_t c0 = 0; c0 < 256u; c0 += 32u) {
+                for (uint32_t c0 = 0; c0 < 128u; c0 += 32u) {
                     uint32_t orow[32];
-                    tmem_ld32(tmem + lane_addr + TC_COL_O + c0, orow);
+                    tmem_ld32(tmem + lane_addr + TC_COL_O + 128u * half + c0, orow);
                     tmem_wait_ld();
 #pragma unroll
-                    for (int c = 0; c < 32; c += 2)
-                        *reinterpret_cast<float2 *>(ps + 2u + c0 + c) = make_float2(__uint_as_float(orow[c]), __uint_as_float(orow[c + 1]));
+                    for (int c = 0; c < 32; c += 4)
+                        *reinterpret_cast<uint4 *>(ps + ((size_t)((128u * half + c0 + c) >> 2) * 128u + row) * 4u) =
+                            make_uint4(orow[c], orow[c + 1], orow[c + 2], orow[c + 3]);
                 }
-                tc_bar_sync(); // every row of the partial is written
-                if (row == 0u) {
-                    fence_acq_rel_gpu(); // release: the partial before the ticket; acquire: the other parts after it
-                    sh->ticket = atomicAdd(counters + sg.item, 1u);
-                    fence_acq_rel_gpu();
-                }
-                tc_bar_sync();
-                if (sh->ticket == sg.npieces - 1u) {
-                    if (row == 0u) counters[sg.item] = 0u; // every part has arrived: ready for the next launch
-                    // merge in index order, this part's own partial included (read back like the others), so that the
-                    // result does not depend on which part came last
-                    float M = NEG_BIG, l = 0.0f;
-                    for (uint32_t pc = 0; pc < sg.npieces; pc++)
-                        M = fmaxf(M, __ldcg(scratch + pf_slot(sg.cta0, pc) * TC_PART + (size_t)row * REC));
-                    float dst_acc[32];
-                    float *dst = out + (size_t)tok * 4096u + (size_t)head * 256u;
-                    for (uint32_t pc = 0; pc < sg.npieces; pc++) {
-                        const float2 ml = __ldcg(reinterpret_cast<const float2 *>(scratch + pf_slot(sg.cta0, pc) * TC_PART + (size_t)row * REC));
-                        l += ml.y * (ml.x > NEG_TEST ? exp2f(ml.x - M) : 0.0f);
-                    }
-                    const float inv = 1.0f / l;
-#pragma unroll 1
-                    for (uint32_t c0 = 0; c0 < 256u; c0 += 32u) {
-#pragma unroll
-                        for (int c = 0; c < 32; c++) dst_acc[c] = 0.0f;
-                        for (uint32_t pc = 0; pc < sg.npieces; pc++) {
-                            const float *pp = scratch + pf_slot(sg.cta0, pc) * TC_PART + (size_t)row * REC;
-                            const float mq = __ldcg(pp);
-                            const float e = mq > NEG_TEST ? exp2f(mq - M) : 0.0f;
-#pragma unroll
-                            for (int c = 0; c < 32; c += 2) {
-                                const float2 v = __ldcg(reinterpret_cast<const float2 *>(pp + 2u + c0 + c));
-                                dst_acc[c] = fmaf(e, v.x, dst_acc[c]);
-                                dst_acc[c + 1] = fmaf(e, v.y, dst_acc[c + 1]);
-                            }
-                        }
-                        if (tok < ntok) {
-#pragma unroll
-                            for (int c = 0; c < 32; c += 4)
-                                *reinterpret_cast<float4 *>(dst + c0 + c) =
-                                    make_float4(dst_acc[c] * inv, dst_acc[c + 1] * inv, dst_acc[c + 2] * inv, dst_acc[c + 3] * inv);
-                        }
-                    }
-                }
-                tc_bar_sync(); // sh->ticket is free for the next segment
             }
-            return true;
-        });
+            tc_fence_before();
+            pair_bar_sync(1u + q4); // red[] is free for the next segment
+            sg = nx;
+        }
     }
 
-    // ---------------- teardown: nothing of this CTA may still be in flight, then free the tensor memory ----------------
+    // ---------------- teardown: nothing of the pair may still be in flight, then free the tensor memory ----------------
     tc_fence_before();
-    __syncthreads();
-    if (sh->abort && tid == 0) {
-        // a wait ran out somewhere: give copies already issued into this CTA's shared memory a bounded time to land
-        for (int s = 0; s < TC_NST; s++) mbar_wait_bounded(bar_kv_full + 8u * s, 0, 200000000ll);
+    __syncwarp();
+    if (sh->abort) { // a wait ran out somewhere: give copies already issued into this CTA's shared memory time to land
+        const long long t0 = clock64();
+        while (clock64() - t0 < 200000000ll) __nanosleep(1000);
     }
-    __syncthreads();
+    cluster_sync();
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem, TC_COLS);
+        tmem_dealloc2(tmem, TC_COLS);
+    }
+}
+
+// Merges the parts of split items: out = sum_s e^(m_s - M) O_s / sum_s e^(m_s - M) l_s, in index order, so that the result
+// does not depend on timing. One block = 32 rows and a quarter of the dims of one CTA's half of an item; a lane's row is
+// fixed, so its weights are worked out once; the output rows leave through shared memory, 256 contiguous bytes each.
+__global__ void __launch_bounds__(256)
+prefill_merge_kernel(const __grid_constant__ PfPlan plan, const float *__restrict__ scratch, float *__restrict__ out) {
+    __shared__ float4 tile[32][17];
+    pdl_launch_dependents();
+    const uint32_t item = blockIdx.y, cta = blockIdx.x >> 4, q4 = (blockIdx.x >> 2) & 3u, quarter = blockIdx.x & 3u;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, row = 32u * q4 + lane;
+    uint32_t base = 0;
+    for (uint32_t i = 0; i < item; i++) base += plan.tiles_of(i);
+    const uint32_t n = plan.tiles_of(item), p0 = base / plan.len, np = (base + n - 1u) / plan.len - p0 + 1u;
+    const uint32_t tok0 = (plan.ngroups - 1u - (item >> 1)) * 32u + 16u * cta;
+    if (np == 1u || tok0 >= plan.ntok) return; // written by the attention kernel, or padding
+    pdl_wait();
+    // the maximum over the parts: eight loads in flight at a time (one at a time, 36 parts took 25 us)
+    float M = NEG_BIG, l = 0.0f;
+    for (uint32_t s0 = 0; s0 < np; s0 += 8u) {
+        float m[8];
+#pragma unroll
+        for (uint32_t i = 0; i < 8u; i++) {
+            const uint32_t s = min(s0 + i, np - 1u);
+            m[i] = __ldcg(scratch + pf_slot(p0 + s, s, cta) * TC_PART + 128u * 256u + 2u * row);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i++) M = fmaxf(M, m[i]);
+    }
+    float4 acc[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+#pragma unroll 4
+    for (uint32_t s = 0; s < np; s++) {
+        const float *ps = scratch + pf_slot(p0 + s, s, cta) * TC_PART;
+        const float2 ml = __ldcg(reinterpret_cast<const float2 *>(ps + 128u * 256u + 2u * row));
+        float4 v[2];
+#pragma unroll
+        for (uint32_t i = 0; i < 2u; i++) v[i] = __ldcg(reinterpret_cast<const float4 *>(ps + ((size_t)(16u * quarter + warp + 8u * i) * 128u + row) * 4u));
+        const float e = ml.x > NEG_TEST ? exp2f(ml.x - M) : 0.0f;
+        l += e * ml.y;
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            acc[i].x = fmaf(e, v[i].x, acc[i].x);
+            acc[i].y = fmaf(e, v[i].y, acc[i].y);
+            acc[i].z = fmaf(e, v[i].z, acc[i].z);
+            acc[i].w = fmaf(e, v[i].w, acc[i].w);
+        }
+    }
+    const float inv = 1.0f / l;
+#pragma unroll
+    for (uint32_t i = 0; i < 2u; i++) tile[lane][warp + 8u * i] = make_float4(acc[i].x * inv, acc[i].y * inv, acc[i].z * inv, acc[i].w * inv);
+    __syncthreads();
+    const uint32_t c = threadIdx.x & 15u;
+#pragma unroll
+    for (uint32_t i = 0; i < 2u; i++) {
+        const uint32_t r = (threadIdx.x >> 4) + 16u * i, rr = 32u * q4 + r, tok = tok0 + (rr & 15u), head = 8u * (item & 1u) + (rr >> 4);
+        if (tok < plan.ntok) *reinterpret_cast<float4 *>(out + (size_t)tok * 4096u + head * 256u + quarter * 64u + 4u * c) = tile[r][c];
     }
 }
 
@@ -482,17 +535,16 @@ mkv_status prefill_tc_setup_device() {
     return MKV_OK;
 }
 
-// Scratch of the split items: two partials per CTA and one arrival counter per item, allocated with the context's
-// first prefill launch that needs them and kept until the context goes.
+// Scratch of the split items: two partials per CTA, allocated with the context's first prefill launch and kept until the
+// context goes.
 static mkv_status prefill_scratch(Ctx *ctx) {
     if (ctx->pf_scratch) return MKV_OK;
     const size_t bytes = 2u * (size_t)ctx->sm_count * TC_PART * sizeof(float);
-    if (cudaMalloc(&ctx->pf_scratch, bytes) != cudaSuccess || cudaMalloc(&ctx->pf_counters, TC_MAX_ITEMS * sizeof(uint32_t)) != cudaSuccess) {
+    if (cudaMalloc(&ctx->pf_scratch, bytes) != cudaSuccess) {
         cudaGetLastError();
         set_error("out of device memory for the prefill partials (%zu bytes)", bytes);
         return MKV_ERR_NOMEM;
     }
-    MKV_CUDA(cudaMemsetAsync(ctx->pf_counters, 0, TC_MAX_ITEMS * sizeof(uint32_t), ctx->stream));
     return MKV_OK;
 }
 
@@ -503,32 +555,47 @@ mkv_status launch_prefill_f16_tc(Ctx *ctx, Cache *c, int layer, uint32_t first_p
 #else
     const uint32_t phase = 0u;
 #endif
-    const uint32_t nitems = 2u * ((ntok + 15u) / 16u);
-    if (nitems > TC_MAX_ITEMS) {
-        set_error("a prefill block of %u tokens is %u work items, at most %u are built", ntok, nitems, TC_MAX_ITEMS);
-        return MKV_ERR_INVALID;
-    }
-    // tiles of all items (the host's copy of PfWork::tiles_of)
-    uint64_t tiles = 0;
-    for (uint32_t grp = 0; grp < nitems / 2u; grp++)
-        tiles += 2ull * ((pos0 + 1u + std::min(grp * 16u + 15u, ntok - 1u) + TC_TILE - 1u) / TC_TILE - first_pos / TC_TILE);
-    // MKV_PREFILL_SPLIT=0 keeps one CTA per item (the schedule the persistent grid is measured against)
-    static const bool allow_split = [] { const char *e = getenv("MKV_PREFILL_SPLIT"); return !(e && e[0] == '0'); }();
-    const bool split = allow_split && 4u * nitems <= 3u * (uint32_t)ctx->sm_count && tiles >= 4ull * (uint64_t)ctx->sm_count;
-    const uint32_t grid = split ? (uint32_t)ctx->sm_count : nitems;
-    if (split) {
-        mkv_status st = prefill_scratch(ctx);
-        if (st != MKV_OK) return st;
-    }
+    PfPlan plan;
+    plan.first_pos = first_pos; plan.pos0 = pos0; plan.ntok = ntok;
+    plan.ngroups = (ntok + 31u) / 32u;
+    plan.nitems = 2u * plan.ngroups;
+    plan.t0 = first_pos / TC_TILE;
+    plan.total = 0;
+    for (uint32_t i = 0; i < plan.nitems; i += 2u) plan.total += 2u * plan.tiles_of(i);
+    const uint32_t npairs = (uint32_t)ctx->sm_count / 2u;
+    plan.len = std::max((plan.total + npairs - 1u) / npairs, TC_MIN_LEN);
+    const uint32_t pairs = (plan.total + plan.len - 1u) / plan.len;
+    mkv_status st = prefill_scratch(ctx);
+    if (st != MKV_OK) return st;
     const CUtensorMap &km = c->maps_host[2 * (c->n_layers + layer)], &vm = c->maps_host[2 * (c->n_layers + layer) + 1];
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2u * pairs);
+    cfg.blockDim = dim3(TC_THREADS);
+    cfg.dynamicSmemBytes = TC_SMEM;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = ctx->pdl ? 1 : 0;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
     if (q_is_f16)
-        prefill_f16_tc_kernel<true><<<grid, 192, TC_SMEM, ctx->stream>>>(km, vm, q, out, first_pos, pos0, ntok, c->shard_first,
-                                                                         ctx->pf_scratch, ctx->pf_counters, split ? 1u : 0u, ctx->dev_status, phase);
+        MKV_CUDA(cudaLaunchKernelEx(&cfg, prefill_f16_tc_kernel<true>, km, vm, q, out, plan, c->shard_first, ctx->pf_scratch, ctx->dev_status, phase));
     else
-        prefill_f16_tc_kernel<false><<<grid, 192, TC_SMEM, ctx->stream>>>(km, vm, q, out, first_pos, pos0, ntok, c->shard_first,
-                                                                          ctx->pf_scratch, ctx->pf_counters, split ? 1u : 0u, ctx->dev_status, phase);
+        MKV_CUDA(cudaLaunchKernelEx(&cfg, prefill_f16_tc_kernel<false>, km, vm, q, out, plan, c->shard_first, ctx->pf_scratch, ctx->dev_status, phase));
     ctx->launches++;
-    MKV_CUDA(cudaGetLastError());
+    bool split = false;
+    for (uint32_t i = 0, base = 0; i < plan.nitems && !split; i++) {
+        const uint32_t n = plan.tiles_of(i);
+        split = base / plan.len != (base + n - 1u) / plan.len;
+        base += n;
+    }
+    if (split) {
+        cfg.gridDim = dim3(32u, plan.nitems);
+        cfg.blockDim = dim3(256);
+        cfg.dynamicSmemBytes = 0;
+        MKV_CUDA(cudaLaunchKernelEx(&cfg, prefill_merge_kernel, plan, (const float *)ctx->pf_scratch, out));
+        ctx->launches++;
+    }
     return MKV_OK;
 }
 

@@ -704,6 +704,27 @@ def test_prefill_over_cache(ctx, oracle, fmt, prefix, ntok, first):
     cache.close()
 
 
+@pytest.mark.parametrize("prefix,ntok,first,q16", [(0, 1, 0, False), (127, 1, 0, True), (126, 33, 0, False), (128, 31, 0, True),
+                                                    (255, 32, 128, False), (383, 65, 129, True), (8100, 5, 0, False), (12000, 40, 11903, False),
+                                                    (15000, 97, 0, True)])
+def test_prefill_f16_tile_and_split_edges(ctx, oracle, prefix, ntok, first, q16):
+    """The f16 prefill kernel at the edges of its key tiles (128), token groups (32 a pair of CTAs, 16 a CTA) and of the split of
+    its work: one tile in all, items of one part, items cut into dozens of parts (few tokens over a long prefix)."""
+    fmt = kv.KvFormat.F16
+    cache = kv.KvCache(ctx, fmt, 1, (prefix + ntok + 4096) // 1024 * 1024)
+    kc, vc = fill_both(oracle, cache, 0, prefix + ntok, 300 + ntok)
+    q = synth.normal(301, synth.S_Q, ntok, (ntok, 16, 256))
+    out = torch.full((ntok + 1, 16, 256), float("nan"), device="cuda")
+    cache.attn_prefill(0, first, prefix, dev(q).half() if q16 else dev(q), out[:ntok])
+    ctx.sync()
+    got = out.cpu().numpy()
+    assert np.isnan(got[ntok]).all()  # nothing past the block is written
+    toks = sorted(set([0, 1, 15, 16, 31, 32, ntok // 2, ntok - 2, ntok - 1]) & set(range(ntok)))
+    want = oracle.attn_ref_f32_sel(int(fmt), kc, vc, first, prefix, toks, q)
+    assert np.isfinite(got[:ntok]).all() and oracle.max_rel(got[toks], want) < TOL[fmt]
+    cache.close()
+
+
 # ---------------------------------------------------------------- snapshot / restore ---------------------------
 
 @pytest.mark.parametrize("fmt", FMTS)
