@@ -268,34 +268,51 @@ prefill_f16_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(bar);
         };
-        // Q of an item goes to tensor memory as the A operand of S = Q K^T (q_f16 of the reference, W/fa_mx.wgsl:313-319):
-        // a row's thread converts 128 of its 256 values to f16 and stores them in its lane, two per 32-bit column.
+        // This warp's own 4 KB of the P buffer (its rows, its 64 keys) is where rows change hands between "a lane has a row" (tensor
+        // memory) and "a few lanes share a row" (coalesced global accesses): free whenever the products so far have completed.
+        uint8_t *stage = smem + TC_OFF_P + 16384u * half + 4096u * q4;
+        // Q of an item goes to tensor memory as the A operand of S = Q K^T (q_f16 of the reference, W/fa_mx.wgsl:313-319), as
+        // f16, two values per 32-bit column: the warp loads 64 dims of its 32 rows at a time, whole lines, and a lane stores its
+        // row. (With every lane loading its own row straight from global memory this took 8 us of a segment for f32 queries
+        // and 3 us for f16 ones.)
         auto load_q = [&](const PfSegment &sg) {
-            const uint32_t tok = (plan.ngroups - 1u - (sg.item >> 1)) * 32u + 16u * cta + (row & 15u), head = 8u * (sg.item & 1u) + (row >> 4);
-            const size_t qoff = (size_t)min(tok, plan.ntok - 1u) * 4096u + (size_t)head * 256u + 128u * half;
+            const uint32_t t0 = (plan.ngroups - 1u - (sg.item >> 1)) * 32u + 16u * cta, h0 = 8u * (sg.item & 1u) + 2u * q4;
+            auto src_of = [&](uint32_t r) { // element offset of the warp's row r (= head * 16 + token), this half's first dim
+                return (size_t)min(t0 + (r & 15u), plan.ntok - 1u) * 4096u + (size_t)(h0 + (r >> 4)) * 256u + 128u * half;
+            };
+            constexpr int NL = QF16 ? 8 : 16; // 16-byte loads of a lane per 64 dims
+            uint4 v[2][NL];
 #pragma unroll
-            for (uint32_t c0 = 0; c0 < 2u; c0++) { // 64 dims = 32 columns per store
-                uint32_t w[32];
-                if constexpr (QF16) { // already f16: eight 16-byte loads per 64 dims
-                    const uint4 *src = reinterpret_cast<const uint4 *>(static_cast<const __half *>(q) + qoff + c0 * 64u);
+            for (int c0 = 0; c0 < 2; c0++)
 #pragma unroll
-                    for (int i = 0; i < 8; i++) {
-                        const uint4 a = src[i];
-                        w[4 * i] = a.x; w[4 * i + 1] = a.y; w[4 * i + 2] = a.z; w[4 * i + 3] = a.w;
-                    }
-                } else {
-                    const float *src = static_cast<const float *>(q) + qoff + c0 * 64u;
+                for (int i = 0; i < NL; i++) {
+                    const uint32_t r = QF16 ? 4u * i + (lane >> 3) : 2u * i + (lane >> 4);
+                    const void *src = QF16 ? static_cast<const void *>(static_cast<const __half *>(q) + src_of(r) + 64u * c0 + 8u * (lane & 7u))
+                                           : static_cast<const void *>(static_cast<const float *>(q) + src_of(r) + 64u * c0 + 4u * (lane & 15u));
+                    v[c0][i] = __ldg(static_cast<const uint4 *>(src));
+                    if (t0 + (r & 15u) >= plan.ntok) v[c0][i] = make_uint4(0u, 0u, 0u, 0u);
+                }
 #pragma unroll
-                    for (int i = 0; i < 16; i++) {
-                        const float4 a = *reinterpret_cast<const float4 *>(src + 4 * i);
-                        const __half2 h0 = __floats2half2_rn(a.x, a.y), h1 = __floats2half2_rn(a.z, a.w);
-                        w[2 * i] = *reinterpret_cast<const uint32_t *>(&h0);
-                        w[2 * i + 1] = *reinterpret_cast<const uint32_t *>(&h1);
+            for (int c0 = 0; c0 < 2; c0++) {
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < NL; i++) {
+                    const uint4 a = v[c0][i];
+                    if constexpr (QF16) {
+                        *reinterpret_cast<uint4 *>(stage + swz128(4u * i + (lane >> 3), lane & 7u)) = a;
+                    } else {
+                        const __half2 h0 = __floats2half2_rn(__uint_as_float(a.x), __uint_as_float(a.y));
+                        const __half2 h1 = __floats2half2_rn(__uint_as_float(a.z), __uint_as_float(a.w));
+                        *reinterpret_cast<uint2 *>(stage + swz128(2u * i + (lane >> 4), (lane & 15u) >> 1) + 8u * (lane & 1u)) =
+                            make_uint2(*reinterpret_cast<const uint32_t *>(&h0), *reinterpret_cast<const uint32_t *>(&h1));
                     }
                 }
-                if (tok >= plan.ntok) {
+                __syncwarp();
+                uint32_t w[32];
 #pragma unroll
-                    for (int i = 0; i < 32; i++) w[i] = 0u;
+                for (uint32_t c = 0; c < 8u; c++) {
+                    const uint4 a = *reinterpret_cast<const uint4 *>(stage + swz128(lane, c));
+                    w[4 * c] = a.x; w[4 * c + 1] = a.y; w[4 * c + 2] = a.z; w[4 * c + 3] = a.w;
                 }
                 tmem_st32(tmem + lane_addr + TC_COL_Q + 64u * half + 32u * c0, w);
             }
@@ -310,8 +327,7 @@ prefill_f16_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
         if (more) load_q(sg);
         while (more) {
             const uint32_t tok0 = (plan.ngroups - 1u - (sg.item >> 1)) * 32u + 16u * cta, kvh = sg.item & 1u;
-            const uint32_t tok = tok0 + (row & 15u), head = 8u * kvh + (row >> 4);
-            const uint32_t vis = plan.pos0 + 1u + tok;         // the row's token sees keys < vis
+            const uint32_t vis = plan.pos0 + 1u + tok0 + (row & 15u); // the row's token sees keys < vis
             const uint32_t full_below = plan.pos0 + 1u + tok0; // keys below this are visible to every row of the CTA
             float m_ref = NEG_BIG, l_run = 0.0f; // l_run: this thread's 64 keys of every tile only
             const uint32_t n = sg.b - sg.a;
@@ -410,31 +426,35 @@ prefill_f16_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
                 tc_fence_before();
                 arrive(r_p_full);
             }
-            // All scores of the segment are there, so its Q may be replaced: the next segment's first scores are computed while
-            // this one's last products and its epilogue run.
-            more = ok && walk.next(nx);
-            if (more) load_q(nx);
             // ---------------- end of the segment: all its MMAs have completed ----------------
             ok = ok && __all_sync(0xffffffffu, tc_wait(bar_pv_done, (g - 1u) & 1u, sh, status));
             tc_fence_after();
+            more = ok && walk.next(nx);
+            if (more) load_q(nx); // the next segment's first scores are computed while this one's epilogue runs
             red[128u * half + row] = l_run;
             if (pair_bar_or(1u + q4, !ok)) break;
             const float l_all = red[row] + red[128u + row];
             if (sg.npieces == 1u) {
                 // the whole item: out[tok][head][:] = O / l
                 const float inv = 1.0f / l_all;
-                float *dst = out + (size_t)tok * 4096u + (size_t)head * 256u + 128u * half;
 #pragma unroll 1
                 for (uint32_t c0 = 0; c0 < 128u; c0 += 32u) {
                     uint32_t orow[32];
                     tmem_ld32(tmem + lane_addr + TC_COL_O + 128u * half + c0, orow);
                     tmem_wait_ld();
-                    if (tok < plan.ntok) {
+                    __syncwarp();
 #pragma unroll
-                        for (int c = 0; c < 32; c += 4)
-                            *reinterpret_cast<float4 *>(dst + c0 + c) =
-                                make_float4(__uint_as_float(orow[c]) * inv, __uint_as_float(orow[c + 1]) * inv,
-                                            __uint_as_float(orow[c + 2]) * inv, __uint_as_float(orow[c + 3]) * inv);
+                    for (uint32_t c = 0; c < 8u; c++)
+                        *reinterpret_cast<float4 *>(stage + swz128(lane, c)) =
+                            make_float4(__uint_as_float(orow[4 * c]) * inv, __uint_as_float(orow[4 * c + 1]) * inv,
+                                        __uint_as_float(orow[4 * c + 2]) * inv, __uint_as_float(orow[4 * c + 3]) * inv);
+                    __syncwarp();
+#pragma unroll
+                    for (uint32_t i = 0; i < 8u; i++) { // eight lanes write a row's 128 bytes
+                        const uint32_t r = 4u * i + (lane >> 3), t = tok0 + (r & 15u), h = 8u * kvh + 2u * q4 + (r >> 4);
+                        if (t < plan.ntok)
+                            *reinterpret_cast<float4 *>(out + (size_t)t * 4096u + h * 256u + 128u * half + c0 + 4u * (lane & 7u)) =
+                                *reinterpret_cast<const float4 *>(stage + swz128(r, lane & 7u));
                     }
                 }
             } else {
@@ -472,61 +492,84 @@ prefill_f16_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
     }
 }
 
-// Merges the parts of split items: out = sum_s e^(m_s - M) O_s / sum_s e^(m_s - M) l_s, in index order, so that the result
-// does not depend on timing. One block = 32 rows and a quarter of the dims of one CTA's half of an item; a lane's row is
-// fixed, so its weights are worked out once; the output rows leave through shared memory, 256 contiguous bytes each.
+// Merges the parts of split items: out = sum_s e^(m_s - M) O_s / sum_s e^(m_s - M) l_s, in a fixed order, so that the result
+// does not depend on timing. One block = 32 rows (one per lane) and an eighth of the dims of one CTA's half of an item; four
+// groups of two warps take every fourth part each (with the maximum of their own parts; the loads of four parts are in flight
+// at once, which is what bounds this kernel: an item of few tokens over a long prefix has dozens of parts) and meet in shared
+// memory, from where the output rows leave as whole lines.
 __global__ void __launch_bounds__(256)
 prefill_merge_kernel(const __grid_constant__ PfPlan plan, const float *__restrict__ scratch, float *__restrict__ out) {
-    __shared__ float4 tile[32][17];
+    __shared__ float2 ml_s[4][32];
+    __shared__ float4 acc_s[4][32][9];
     pdl_launch_dependents();
-    const uint32_t item = blockIdx.y, cta = blockIdx.x >> 4, q4 = (blockIdx.x >> 2) & 3u, quarter = blockIdx.x & 3u;
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, row = 32u * q4 + lane;
+    const uint32_t item = blockIdx.y, cta = blockIdx.x >> 5, q4 = (blockIdx.x >> 3) & 3u, eighth = blockIdx.x & 7u;
+    const uint32_t lane = threadIdx.x & 31u, grp = threadIdx.x >> 6, ch = (threadIdx.x >> 5) & 1u, row = 32u * q4 + lane;
     uint32_t base = 0;
     for (uint32_t i = 0; i < item; i++) base += plan.tiles_of(i);
     const uint32_t n = plan.tiles_of(item), p0 = base / plan.len, np = (base + n - 1u) / plan.len - p0 + 1u;
     const uint32_t tok0 = (plan.ngroups - 1u - (item >> 1)) * 32u + 16u * cta;
     if (np == 1u || tok0 >= plan.ntok) return; // written by the attention kernel, or padding
     pdl_wait();
-    // the maximum over the parts: eight loads in flight at a time (one at a time, 36 parts took 25 us)
     float M = NEG_BIG, l = 0.0f;
-    for (uint32_t s0 = 0; s0 < np; s0 += 8u) {
-        float m[8];
+    float4 acc[4];
 #pragma unroll
-        for (uint32_t i = 0; i < 8u; i++) {
-            const uint32_t s = min(s0 + i, np - 1u);
-            m[i] = __ldcg(scratch + pf_slot(p0 + s, s, cta) * TC_PART + 128u * 256u + 2u * row);
+    for (int i = 0; i < 4; i++) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (uint32_t s0 = grp; s0 < np; s0 += 16u) {
+        float2 ml[4];
+        float4 v[4][4];
+#pragma unroll
+        for (uint32_t k = 0; k < 4u; k++) {
+            const uint32_t s = s0 + 4u * k;
+            const float *ps = scratch + pf_slot(p0 + min(s, np - 1u), s, cta) * TC_PART; // (s > 0 from the second part on)
+            ml[k] = s < np ? __ldcg(reinterpret_cast<const float2 *>(ps + 128u * 256u + 2u * row)) : make_float2(NEG_BIG, 0.0f);
+#pragma unroll
+            for (uint32_t i = 0; i < 4u; i++)
+                v[k][i] = s < np ? __ldcg(reinterpret_cast<const float4 *>(ps + ((size_t)(8u * eighth + 4u * ch + i) * 128u + row) * 4u))
+                                 : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        const float mx = fmaxf(fmaxf(ml[0].x, ml[1].x), fmaxf(ml[2].x, ml[3].x));
+        if (mx > M) {
+            const float f = M > NEG_TEST ? exp2f(M - mx) : 0.0f;
+            l *= f;
+#pragma unroll
+            for (int i = 0; i < 4; i++) acc[i] = make_float4(acc[i].x * f, acc[i].y * f, acc[i].z * f, acc[i].w * f);
+            M = mx;
         }
 #pragma unroll
-        for (int i = 0; i < 8; i++) M = fmaxf(M, m[i]);
-    }
-    float4 acc[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
-#pragma unroll 4
-    for (uint32_t s = 0; s < np; s++) {
-        const float *ps = scratch + pf_slot(p0 + s, s, cta) * TC_PART;
-        const float2 ml = __ldcg(reinterpret_cast<const float2 *>(ps + 128u * 256u + 2u * row));
-        float4 v[2];
+        for (int k = 0; k < 4; k++) {
+            const float e = ml[k].x > NEG_TEST ? exp2f(ml[k].x - M) : 0.0f;
+            l = fmaf(e, ml[k].y, l);
 #pragma unroll
-        for (uint32_t i = 0; i < 2u; i++) v[i] = __ldcg(reinterpret_cast<const float4 *>(ps + ((size_t)(16u * quarter + warp + 8u * i) * 128u + row) * 4u));
-        const float e = ml.x > NEG_TEST ? exp2f(ml.x - M) : 0.0f;
-        l += e * ml.y;
-#pragma unroll
-        for (int i = 0; i < 2; i++) {
-            acc[i].x = fmaf(e, v[i].x, acc[i].x);
-            acc[i].y = fmaf(e, v[i].y, acc[i].y);
-            acc[i].z = fmaf(e, v[i].z, acc[i].z);
-            acc[i].w = fmaf(e, v[i].w, acc[i].w);
+            for (int i = 0; i < 4; i++) {
+                acc[i].x = fmaf(e, v[k][i].x, acc[i].x);
+                acc[i].y = fmaf(e, v[k][i].y, acc[i].y);
+                acc[i].z = fmaf(e, v[k][i].z, acc[i].z);
+                acc[i].w = fmaf(e, v[k][i].w, acc[i].w);
+            }
         }
     }
-    const float inv = 1.0f / l;
+    if (ch == 0u) ml_s[grp][lane] = make_float2(M, l);
 #pragma unroll
-    for (uint32_t i = 0; i < 2u; i++) tile[lane][warp + 8u * i] = make_float4(acc[i].x * inv, acc[i].y * inv, acc[i].z * inv, acc[i].w * inv);
+    for (uint32_t i = 0; i < 4u; i++) acc_s[grp][lane][4u * ch + i] = acc[i];
     __syncthreads();
-    const uint32_t c = threadIdx.x & 15u;
+    const uint32_t r = threadIdx.x >> 3, c = threadIdx.x & 7u, rr = 32u * q4 + r, tok = tok0 + (rr & 15u);
+    if (tok >= plan.ntok) return;
+    const float Mr = fmaxf(fmaxf(ml_s[0][r].x, ml_s[1][r].x), fmaxf(ml_s[2][r].x, ml_s[3][r].x));
+    float L = 0.0f;
+    float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (uint32_t i = 0; i < 2u; i++) {
-        const uint32_t r = (threadIdx.x >> 4) + 16u * i, rr = 32u * q4 + r, tok = tok0 + (rr & 15u), head = 8u * (item & 1u) + (rr >> 4);
-        if (tok < plan.ntok) *reinterpret_cast<float4 *>(out + (size_t)tok * 4096u + head * 256u + quarter * 64u + 4u * c) = tile[r][c];
+    for (int g = 0; g < 4; g++) {
+        const float e = ml_s[g][r].x > NEG_TEST ? exp2f(ml_s[g][r].x - Mr) : 0.0f;
+        const float4 a = acc_s[g][r][c];
+        L = fmaf(e, ml_s[g][r].y, L);
+        y.x = fmaf(e, a.x, y.x);
+        y.y = fmaf(e, a.y, y.y);
+        y.z = fmaf(e, a.z, y.z);
+        y.w = fmaf(e, a.w, y.w);
     }
+    const float inv = 1.0f / L;
+    *reinterpret_cast<float4 *>(out + (size_t)tok * 4096u + (8u * (item & 1u) + (rr >> 4)) * 256u + 32u * eighth + 4u * c) =
+        make_float4(y.x * inv, y.y * inv, y.z * inv, y.w * inv);
 }
 
 mkv_status prefill_tc_setup_device() {
@@ -590,7 +633,7 @@ mkv_status launch_prefill_f16_tc(Ctx *ctx, Cache *c, int layer, uint32_t first_p
         base += n;
     }
     if (split) {
-        cfg.gridDim = dim3(32u, plan.nitems);
+        cfg.gridDim = dim3(64u, plan.nitems);
         cfg.blockDim = dim3(256);
         cfg.dynamicSmemBytes = 0;
         MKV_CUDA(cudaLaunchKernelEx(&cfg, prefill_merge_kernel, plan, (const float *)ctx->pf_scratch, out));
