@@ -26,6 +26,8 @@ mkv_status prefill_setup_device();
 mkv_status prefill_tc_setup_device();
 mkv_status launch_prefill_f16_tc(Ctx *ctx, Cache *c, int layer, uint32_t first_pos, uint32_t pos0, uint32_t ntok,
                                  const void *q, bool q_is_f16, float *out);
+mkv_status prefill_f32_tc_setup_device();
+mkv_status launch_prefill_f32_tc(Ctx *ctx, Cache *c, int layer, uint32_t first_pos, uint32_t pos0, uint32_t ntok, const float *q, float *out);
 mkv_status launch_q_f16(Ctx *ctx, const float *src, void *dst, size_t n_pairs);
 mkv_status append_setup_device();
 mkv_status launch_prefill_f16_mma(Ctx *ctx, Cache *c, int layer, uint32_t first_pos, uint32_t pos0, uint32_t ntok,
@@ -370,6 +372,7 @@ mkv_status mkv_ctx_create(int device, void *stream, mkv_ctx **out) {
     mkv_status st = verify_setup_device();
     if (st == MKV_OK) st = prefill_setup_device();
     if (st == MKV_OK) st = prefill_tc_setup_device();
+    if (st == MKV_OK) st = prefill_f32_tc_setup_device();
     if (st == MKV_OK) st = append_setup_device();
     if (st != MKV_OK) return st;
     *out = reinterpret_cast<mkv_ctx *>(ctx);
@@ -539,12 +542,11 @@ static mkv_status cache_create_common(mkv_ctx *h, mkv_fmt fmt, int n_layers, uin
     std::vector<CUtensorMap> &maps = c->maps_host;
     maps.resize(4 * (size_t)n_layers);
     const uint32_t box_rows = fmt == MKV_F16 ? TILE : TILE32;
-    const uint32_t pf_rows = fmt == MKV_F16 ? PF_TILE : TILE32;
     for (int l = 0; l < n_layers; l++) {
         if ((st = make_tensor_map(&maps[2 * l], fmt, c->k[l], capacity, box_rows)) != MKV_OK) return fail(st);
         if ((st = make_tensor_map(&maps[2 * l + 1], fmt, c->v[l], capacity, box_rows)) != MKV_OK) return fail(st);
-        if ((st = make_tensor_map(&maps[2 * (n_layers + l)], fmt, c->k[l], capacity, pf_rows)) != MKV_OK) return fail(st);
-        if ((st = make_tensor_map(&maps[2 * (n_layers + l) + 1], fmt, c->v[l], capacity, pf_rows)) != MKV_OK) return fail(st);
+        if ((st = make_tensor_map(&maps[2 * (n_layers + l)], fmt, c->k[l], capacity, PF_TILE)) != MKV_OK) return fail(st);
+        if ((st = make_tensor_map(&maps[2 * (n_layers + l) + 1], fmt, c->v[l], capacity, PF_TILE)) != MKV_OK) return fail(st);
     }
     if (cudaMalloc(&c->maps_dev, maps.size() * sizeof(CUtensorMap)) != cudaSuccess ||
         cudaMalloc(&c->kptrs_dev, n_layers * sizeof(void *)) != cudaSuccess ||
@@ -1098,7 +1100,14 @@ mkv_status mkv_attn_prefill(mkv_cache *h, int layer, uint32_t first_pos, uint32_
         set_error("f16 queries go with the f16 cache (q_f16 + attn_fa_mx); the f32 cache's attn_fa / attn_fd4 read f32 queries");
         return MKV_ERR_UNSUPPORTED;
     }
-    // f32 cache: groups of up to 4 tokens through the f32 verify kernel (the reference's attn_fd4 also reads
+    // f32 cache, two ways. prefill_f32_tc.cu takes 32 tokens at a time: about 27 us a layer and 1.3 us per 1,000 keys and 32
+    // tokens. Batched verify items take 4 tokens: about 12 us and 0.65 us per 1,000 keys and 4 tokens, so they win for a few
+    // tokens. Measured, us a layer, items / kernel: 5 tokens over 4,096 16 / 32, 16 over 4,096 22 / 34, 16 over 8,192 33 / 38,
+    // 32 over 4,096 36 / 34, 16 over 32,768 95 / 70, 64 over 1,000 30 / 33, 64 over 4,096 70 / 36, 512 over 4,096 567 / 124.
+    const uint32_t g4 = (ntok + 3u) / 4u, g32 = (ntok + 31u) / 32u;
+    if (g4 > 2u * g32 && (uint64_t)(g4 - 2u * g32) * (end - first_pos) >= 23000u)
+        return launch_prefill_f32_tc(c->ctx, c, layer, first_pos, pos0, ntok, q, out);
+    // groups of up to 4 tokens through the f32 verify kernel (the reference's attn_fd4 also reads
     // K/V once per 4 tokens, W/ops.wgsl:694-699), one ragged batch per <= SLOT_ITEMS groups
     uint32_t done = 0;
     while (done < ntok) {

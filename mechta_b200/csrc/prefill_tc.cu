@@ -34,13 +34,13 @@
 #include <algorithm>
 
 #include "internal.cuh"
+#include "prefill_plan.cuh"
 #include "ptx.cuh"
 
 namespace mkv {
 using namespace ptx;
 
 constexpr int TC_NST = 3;                              // ring depth, K and V each
-constexpr uint32_t TC_TILE = 128;                      // keys per tile
 constexpr uint32_t TC_BOX = 8192;                      // one TMA box [64 keys][64 dims] f16 (PF_TILE rows)
 constexpr uint32_t TC_HALF = 32768;                    // a CTA's half of a K or V tile
 constexpr uint32_t TC_OFF_V = TC_NST * TC_HALF;
@@ -58,10 +58,6 @@ constexpr long long TC_WAIT_LIMIT = 2000000000ll;
 constexpr float TC_LOG2E = 1.4426950408889634f;
 constexpr float TC_LAZY2 = 8.0f * TC_LOG2E;
 constexpr float TC_C2 = SCALE * TC_LOG2E;              // scores to base-2 exponents
-constexpr uint32_t TC_MIN_LEN = 2;                     // tiles a pair takes at least: a shorter range costs more in partials than it saves
-// One partial of a CTA: O as [64 chunks of 4 dims][128 rows][4] (a warp's rows store and load 512 contiguous bytes), then
-// [128 rows][m, l]
-constexpr size_t TC_PART = 128u * 256u + 128u * 2u;
 static_assert(TC_SMEM <= 232448, "shared memory of prefill_f16_tc_kernel");
 
 struct TcShared {
@@ -77,52 +73,6 @@ __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, TcShared 
     sh->abort = 1;
     atomicOr(status, DEV_ERR_WAIT_TIMEOUT);
     return false;
-}
-
-// The work of one launch. Items are numbered longest first: item i = (group of 32 tokens ngroups - 1 - i / 2, KV head i % 2);
-// its tiles are the 128-key tiles from first_pos / 128 up to the last key its last token sees. Pair p takes the tiles
-// [p * len, (p + 1) * len) of all items laid end to end.
-struct PfPlan {
-    uint32_t first_pos, pos0, ntok;
-    uint32_t ngroups, nitems, t0;
-    uint32_t total, len;
-    __host__ __device__ uint32_t tiles_of(uint32_t item) const {
-        const uint32_t grp = ngroups - 1u - (item >> 1);
-        const uint32_t last = grp * 32u + 31u < ntok - 1u ? grp * 32u + 31u : ntok - 1u;
-        return (pos0 + last + TC_TILE) / TC_TILE - t0;
-    }
-};
-struct PfSegment {
-    uint32_t item, a, b;     // tiles [a, b) of the item
-    uint32_t piece, npieces; // which part of the item this is, of how many
-};
-// Walks the segments of one pair.
-struct PfWalk {
-    const PfPlan &p;
-    uint32_t pair, lo, hi, item, base;
-    __device__ __forceinline__ PfWalk(const PfPlan &plan, uint32_t pair_) : p(plan), pair(pair_), item(0), base(0) {
-        lo = min(pair * p.len, p.total);
-        hi = min(lo + p.len, p.total);
-    }
-    __device__ __forceinline__ bool next(PfSegment &s) {
-        while (item < p.nitems && base < hi) {
-            const uint32_t n = p.tiles_of(item), a = max(base, lo), b = min(base + n, hi);
-            if (b > a) {
-                const uint32_t c0 = base / p.len;
-                s = {item, a - base, b - base, pair - c0, (base + n - 1u) / p.len - c0 + 1u};
-            }
-            const bool found = b > a;
-            base += n;
-            item++;
-            if (found) return true;
-        }
-        return false;
-    }
-};
-// Where a pair's CTA keeps the partial of a part: a pair has at most one segment that continues an item begun by the pair
-// before it (slot 0) and at most one that begins an item it does not finish (slot 1).
-__host__ __device__ inline size_t pf_slot(uint32_t pair, uint32_t piece, uint32_t cta) {
-    return ((size_t)pair * 2u + (piece == 0u ? 1u : 0u)) * 2u + cta;
 }
 
 // QF16: the queries come as f16 [ntok][16][256] (the output of the reference's q_f16 pass) instead of f32.
@@ -179,9 +129,9 @@ prefill_f16_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
             bool ok = true;
             while (ok && walk.next(sg)) {
                 const int x = (int)((sg.item & 1u) * 256u);
-                const uint32_t end = plan.pos0 + plan.ntok; // no key at or past this one is seen by anybody
+                const uint32_t end = plan.pos0 + plan.item_end(sg.item); // no key at or past this one is seen by the item's tokens
                 for (uint32_t j = sg.a; j < sg.b; j++, g++) {
-                    const uint32_t s = g % TC_NST, key0 = (plan.t0 + j) * TC_TILE;
+                    const uint32_t s = g % TC_NST, key0 = (plan.t0 + j) * PF_KEYS;
                     const int y[2] = {(int)(key0 - row0), key0 + 64u < end ? (int)(key0 + 64u - row0) : TC_ROW_OUTSIDE};
                     const uint32_t par = ((g / TC_NST) - 1u) & 1u;
                     if (g >= (uint32_t)TC_NST && !(ok = tc_wait(bar_k_empty + 8u * s, par, sh, status))) break;
@@ -276,7 +226,7 @@ prefill_f16_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
         // row. (With every lane loading its own row straight from global memory this took 8 us of a segment for f32 queries
         // and 3 us for f16 ones.)
         auto load_q = [&](const PfSegment &sg) {
-            const uint32_t t0 = (plan.ngroups - 1u - (sg.item >> 1)) * 32u + 16u * cta, h0 = 8u * (sg.item & 1u) + 2u * q4;
+            const uint32_t t0 = plan.group_of(sg.item) * 32u + 16u * cta, h0 = 8u * (sg.item & 1u) + 2u * q4;
             auto src_of = [&](uint32_t r) { // element offset of the warp's row r (= head * 16 + token), this half's first dim
                 return (size_t)min(t0 + (r & 15u), plan.ntok - 1u) * 4096u + (size_t)(h0 + (r >> 4)) * 256u + 128u * half;
             };
@@ -326,7 +276,7 @@ prefill_f16_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
         bool more = walk.next(sg), ok = true;
         if (more) load_q(sg);
         while (more) {
-            const uint32_t tok0 = (plan.ngroups - 1u - (sg.item >> 1)) * 32u + 16u * cta, kvh = sg.item & 1u;
+            const uint32_t tok0 = plan.group_of(sg.item) * 32u + 16u * cta, kvh = sg.item & 1u;
             const uint32_t vis = plan.pos0 + 1u + tok0 + (row & 15u); // the row's token sees keys < vis
             const uint32_t full_below = plan.pos0 + 1u + tok0; // keys below this are visible to every row of the CTA
             float m_ref = NEG_BIG, l_run = 0.0f; // l_run: this thread's 64 keys of every tile only
@@ -350,7 +300,7 @@ prefill_f16_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
                 tmem_wait_ld();
                 tc_fence_before();
                 arrive(r_s_free); // the next tile's scores may be computed
-                const uint32_t key_base = (plan.t0 + sg.a + j) * TC_TILE + 64u * half;
+                const uint32_t key_base = (plan.t0 + sg.a + j) * PF_KEYS + 64u * half;
                 // work in base-2 exponents: exp(s / 16 - m) = 2^(s * C - m2), C = log2(e) / 16, one FFMA + one ex2 per score
                 float mt[4] = {NEG_BIG, NEG_BIG, NEG_BIG, NEG_BIG};
                 if (key_base + 64u > full_below || key_base < plan.first_pos) { // the causal diagonal or the window start (W/fa_mx.wgsl:62)
@@ -459,7 +409,7 @@ prefill_f16_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
                 }
             } else {
                 // a part of an item: its partial goes to scratch memory for the merge kernel
-                float *ps = scratch + pf_slot(pair, sg.piece, cta) * TC_PART;
+                float *ps = scratch + pf_slot(pair, sg.piece, cta) * PF_PART;
                 if (half == 0u) *reinterpret_cast<float2 *>(ps + 128u * 256u + 2u * row) = make_float2(m_ref, l_all);
 #pragma unroll 1
                 for (uint32_t c0 = 0; c0 < 128u; c0 += 32u) {
@@ -507,7 +457,7 @@ prefill_merge_kernel(const __grid_constant__ PfPlan plan, const float *__restric
     uint32_t base = 0;
     for (uint32_t i = 0; i < item; i++) base += plan.tiles_of(i);
     const uint32_t n = plan.tiles_of(item), p0 = base / plan.len, np = (base + n - 1u) / plan.len - p0 + 1u;
-    const uint32_t tok0 = (plan.ngroups - 1u - (item >> 1)) * 32u + 16u * cta;
+    const uint32_t tok0 = plan.group_of(item) * 32u + 16u * cta;
     if (np == 1u || tok0 >= plan.ntok) return; // written by the attention kernel, or padding
     pdl_wait();
     float M = NEG_BIG, l = 0.0f;
@@ -520,7 +470,7 @@ prefill_merge_kernel(const __grid_constant__ PfPlan plan, const float *__restric
 #pragma unroll
         for (uint32_t k = 0; k < 4u; k++) {
             const uint32_t s = s0 + 4u * k;
-            const float *ps = scratch + pf_slot(p0 + min(s, np - 1u), s, cta) * TC_PART; // (s > 0 from the second part on)
+            const float *ps = scratch + pf_slot(p0 + min(s, np - 1u), s, cta) * PF_PART; // (s > 0 from the second part on)
             ml[k] = s < np ? __ldcg(reinterpret_cast<const float2 *>(ps + 128u * 256u + 2u * row)) : make_float2(NEG_BIG, 0.0f);
 #pragma unroll
             for (uint32_t i = 0; i < 4u; i++)
@@ -578,16 +528,49 @@ mkv_status prefill_tc_setup_device() {
     return MKV_OK;
 }
 
-// Scratch of the split items: two partials per CTA, allocated with the context's first prefill launch and kept until the
-// context goes.
-static mkv_status prefill_scratch(Ctx *ctx) {
+mkv_status prefill_scratch(Ctx *ctx) {
     if (ctx->pf_scratch) return MKV_OK;
-    const size_t bytes = 2u * (size_t)ctx->sm_count * TC_PART * sizeof(float);
+    const size_t bytes = 2u * (size_t)ctx->sm_count * PF_PART * sizeof(float);
     if (cudaMalloc(&ctx->pf_scratch, bytes) != cudaSuccess) {
         cudaGetLastError();
         set_error("out of device memory for the prefill partials (%zu bytes)", bytes);
         return MKV_ERR_NOMEM;
     }
+    return MKV_OK;
+}
+
+PfPlan pf_plan(Ctx *ctx, uint32_t first_pos, uint32_t pos0, uint32_t ntok) {
+    PfPlan plan;
+    plan.first_pos = first_pos; plan.pos0 = pos0; plan.ntok = ntok;
+    plan.ngroups = (ntok + 31u) / 32u;
+    plan.nitems = 2u * plan.ngroups;
+    plan.t0 = first_pos / PF_KEYS;
+    plan.total = 0;
+    for (uint32_t i = 0; i < plan.nitems; i += 2u) plan.total += 2u * plan.tiles_of(i);
+    const uint32_t npairs = (uint32_t)ctx->sm_count / 2u;
+    plan.len = std::max((plan.total + npairs - 1u) / npairs, PF_MIN_LEN);
+    return plan;
+}
+
+mkv_status launch_prefill_merge(Ctx *ctx, const PfPlan &plan, float *out) {
+    bool split = false;
+    for (uint32_t i = 0, base = 0; i < plan.nitems && !split; i++) {
+        const uint32_t n = plan.tiles_of(i);
+        split = base / plan.len != (base + n - 1u) / plan.len;
+        base += n;
+    }
+    if (!split) return MKV_OK;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(64u, plan.nitems);
+    cfg.blockDim = dim3(256);
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = ctx->pdl ? 1 : 0;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    MKV_CUDA(cudaLaunchKernelEx(&cfg, prefill_merge_kernel, plan, (const float *)ctx->pf_scratch, out));
+    ctx->launches++;
     return MKV_OK;
 }
 
@@ -598,21 +581,12 @@ mkv_status launch_prefill_f16_tc(Ctx *ctx, Cache *c, int layer, uint32_t first_p
 #else
     const uint32_t phase = 0u;
 #endif
-    PfPlan plan;
-    plan.first_pos = first_pos; plan.pos0 = pos0; plan.ntok = ntok;
-    plan.ngroups = (ntok + 31u) / 32u;
-    plan.nitems = 2u * plan.ngroups;
-    plan.t0 = first_pos / TC_TILE;
-    plan.total = 0;
-    for (uint32_t i = 0; i < plan.nitems; i += 2u) plan.total += 2u * plan.tiles_of(i);
-    const uint32_t npairs = (uint32_t)ctx->sm_count / 2u;
-    plan.len = std::max((plan.total + npairs - 1u) / npairs, TC_MIN_LEN);
-    const uint32_t pairs = (plan.total + plan.len - 1u) / plan.len;
+    const PfPlan plan = pf_plan(ctx, first_pos, pos0, ntok);
     mkv_status st = prefill_scratch(ctx);
     if (st != MKV_OK) return st;
     const CUtensorMap &km = c->maps_host[2 * (c->n_layers + layer)], &vm = c->maps_host[2 * (c->n_layers + layer) + 1];
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2u * pairs);
+    cfg.gridDim = dim3(2u * pf_pairs(plan));
     cfg.blockDim = dim3(TC_THREADS);
     cfg.dynamicSmemBytes = TC_SMEM;
     cfg.stream = ctx->stream;
@@ -626,20 +600,7 @@ mkv_status launch_prefill_f16_tc(Ctx *ctx, Cache *c, int layer, uint32_t first_p
     else
         MKV_CUDA(cudaLaunchKernelEx(&cfg, prefill_f16_tc_kernel<false>, km, vm, q, out, plan, c->shard_first, ctx->pf_scratch, ctx->dev_status, phase));
     ctx->launches++;
-    bool split = false;
-    for (uint32_t i = 0, base = 0; i < plan.nitems && !split; i++) {
-        const uint32_t n = plan.tiles_of(i);
-        split = base / plan.len != (base + n - 1u) / plan.len;
-        base += n;
-    }
-    if (split) {
-        cfg.gridDim = dim3(64u, plan.nitems);
-        cfg.blockDim = dim3(256);
-        cfg.dynamicSmemBytes = 0;
-        MKV_CUDA(cudaLaunchKernelEx(&cfg, prefill_merge_kernel, plan, (const float *)ctx->pf_scratch, out));
-        ctx->launches++;
-    }
-    return MKV_OK;
+    return launch_prefill_merge(ctx, plan, out);
 }
 
 } // namespace mkv
