@@ -8,7 +8,7 @@
 // Scheduling. Every CTA writes its piece and publishes it: the threads that wrote it meet at a barrier, one of
 // them issues a release fence and takes a ticket from a counter in global memory. The last R = min(CTAs of the
 // item, 64) arrivals wait (bounded) until the counter shows that all pieces are there, and each merges a share of
-// the item's 64 rows. Only CTAs that have finished their own work ever wait, and fewer of them than there are SMs,
+// the item's 64 rows (or rows of warps, see finish_item). Only CTAs that have finished their own work ever wait, and fewer of them than there are SMs,
 // so the others always make progress; the earlier arrivals leave at once, which lets the CTAs of the next launch
 // in the stream start on their SMs and load their first tiles.
 // (Measured against this: per-piece flags with merging CTAs that gather the pieces as they land, whole rows or
@@ -144,6 +144,25 @@ __device__ __forceinline__ bool exchange_row(const PushInfo &P, uint32_t epoch, 
     return true;
 }
 
+// Four values (column c4 of 64) of a final output row: the sums `a` times `inv`, times the output gate if there is one.
+__device__ __forceinline__ void store_row(const VerifyItem &it, uint32_t tok, uint32_t head, uint32_t c4, const float4 &a, float inv,
+                                          const float4 &gate) {
+    float4 y = make_float4(a.x * inv, a.y * inv, a.z * inv, a.w * inv);
+    const size_t o = (size_t)tok * 4096u + (size_t)head * 256u + 4u * c4;
+    if (it.gate) { // attn_gate of the reference (W/ops.wgsl:171-177): times the sigmoid of the head's gate values
+        y.x *= 1.0f / (1.0f + expf(-gate.x));
+        y.y *= 1.0f / (1.0f + expf(-gate.y));
+        y.z *= 1.0f / (1.0f + expf(-gate.z));
+        y.w *= 1.0f / (1.0f + expf(-gate.w));
+    }
+    if (it.out) *reinterpret_cast<float4 *>(it.out + o) = y;
+    if (it.out16) { // attn_gate16 (W/ops.wgsl:295-300): the same values as f16
+        const __half2 h0 = __floats2half2_rn(y.x, y.y), h1 = __floats2half2_rn(y.z, y.w);
+        *reinterpret_cast<uint2 *>(static_cast<__half *>(it.out16) + o) =
+            make_uint2(*reinterpret_cast<const uint32_t *>(&h0), *reinterpret_cast<const uint32_t *>(&h1));
+    }
+}
+
 // One row (kvh * 32 + row) of one item, by all NT threads of the CTA; all pieces are in global memory.
 // EXT = false compiles the sink handling out (the kernels of the plain path are instantiated without it).
 template <int NT, bool EXT>
@@ -259,28 +278,63 @@ __device__ __forceinline__ void merge_row(const VerifyItem &it, uint32_t r, Fini
                 if (tid == 0) *reinterpret_cast<float2 *>(rec) = make_float2(M, tot);
             }
         } else {
-            const float inv = 1.0f / tot;
-            float4 y = make_float4(a.x * inv, a.y * inv, a.z * inv, a.w * inv);
-            const size_t o = (size_t)tok * 4096u + (size_t)head * 256u + 4 * tid;
-            if (it.gate) { // attn_gate of the reference (W/ops.wgsl:171-177): times the sigmoid of the head's gate values
-                const float4 g = gate;
-                y.x *= 1.0f / (1.0f + expf(-g.x));
-                y.y *= 1.0f / (1.0f + expf(-g.y));
-                y.z *= 1.0f / (1.0f + expf(-g.z));
-                y.w *= 1.0f / (1.0f + expf(-g.w));
-            }
-            if (it.out) *reinterpret_cast<float4 *>(it.out + o) = y;
-            if (it.out16) { // attn_gate16 (W/ops.wgsl:295-300): the same values as f16
-                const __half2 h0 = __floats2half2_rn(y.x, y.y), h1 = __floats2half2_rn(y.z, y.w);
-                *reinterpret_cast<uint2 *>(static_cast<__half *>(it.out16) + o) =
-                    make_uint2(*reinterpret_cast<const uint32_t *>(&h0), *reinterpret_cast<const uint32_t *>(&h1));
-            }
+            store_row(it, tok, head, tid, a, 1.0f / tot, gate);
         }
     }
     if (it.partial && it.push && !exchange_row<NT>(*it.push, it.push_epoch, tok * 16u + head, it.out, status, sm.red)) {
         if (tid == 0) sm.ok = 0u; // a rank never delivered: the CTA's other rows would only wait as long again
         __syncthreads();
     }
+}
+
+// A row (H = 2) or half a row (H = 1, half `half`) of one item by one warp, for items of few pieces (at most 32; final outputs
+// only): the same sums in index order.
+template <int NT, bool EXT, int H>
+__device__ __forceinline__ void merge_row_warp(const VerifyItem &it, uint32_t kvh, uint32_t row, uint32_t half) {
+    constexpr uint32_t IN_FLIGHT = (NT > 256 ? 8 : 16) / H; // pieces whose loads go out together (as the registers allow)
+    const uint32_t lane = threadIdx.x & 31u, tok = row >> 3, head = 8u * kvh + (row & 7u), ns = it.nsplit, c4 = 32u * half + lane;
+    const float4 *po = reinterpret_cast<const float4 *>(it.part_o + ((size_t)kvh * ns * 32u + row) * 256u) + c4;
+    const float2 ml = lane < ns ? __ldcg(reinterpret_cast<const float2 *>(it.part_ml) + ((size_t)kvh * ns + lane) * 32u + row)
+                                : make_float2(NEG_BIG, 0.0f);
+    float4 gate[H], acc[H];
+#pragma unroll
+    for (int h = 0; h < H; h++) {
+        gate[h] = acc[h] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (it.gate) gate[h] = __ldg(reinterpret_cast<const float4 *>(it.gate + ((size_t)tok * 16u + head) * 512u + 256u) + c4 + 32 * h);
+    }
+    float e = 0.0f, tot = 0.0f;
+    for (uint32_t s0 = 0; s0 < ns; s0 += IN_FLIGHT) {
+        float4 x[IN_FLIGHT][H];
+#pragma unroll
+        for (uint32_t i = 0; i < IN_FLIGHT; i++)
+#pragma unroll
+            for (int h = 0; h < H; h++)
+                x[i][h] = s0 + i < ns ? __ldcg(po + (size_t)(s0 + i) * 2048u + 32 * h) : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (s0 == 0u) {
+            float M = ml.x;
+#pragma unroll
+            for (int sh = 16; sh > 0; sh >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, sh));
+            if (EXT && it.sinks) M = fmaxf(M, it.sinks[head]); // joins the maximum and the sum, never the output
+            e = lane < ns ? expf(ml.x - M) : 0.0f;
+            tot = e * ml.y;
+#pragma unroll
+            for (int sh = 16; sh > 0; sh >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, sh);
+            if (EXT && it.sinks) tot += expf(it.sinks[head] - M);
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < IN_FLIGHT; i++) {
+            const float w = __shfl_sync(0xffffffffu, e, (int)((s0 + i) & 31u)); // 0 from the last piece on
+#pragma unroll
+            for (int h = 0; h < H; h++) {
+                acc[h].x += w * x[i][h].x;
+                acc[h].y += w * x[i][h].y;
+                acc[h].z += w * x[i][h].z;
+                acc[h].w += w * x[i][h].w;
+            }
+        }
+    }
+#pragma unroll
+    for (int h = 0; h < H; h++) store_row(it, tok, head, c4 + 32u * h, acc[h], 1.0f / tot, gate[h]);
 }
 
 // The CTA's share of the merge, given its ticket (publish_piece). Called by every thread of every CTA of an item;
@@ -314,8 +368,23 @@ __device__ __forceinline__ void finish_item(const VerifyItem &it, FinishSmem &sm
     }
     __syncthreads(); // thread 0's acquire, passed on by the barrier, orders the piece loads (which bypass L1) behind the publications
     if (!sm.ok) return;
-    for (uint32_t r = ticket - (total - R); r < FIN_JOBS; r += R) {
-        merge_row<NT, EXT>(it, r, sm, status);
+    // Fewer CTAs than the item has rows: job j is row j / 2 of KV head j % 2, so that the rows of a step of few tokens do not
+    // meet in the same CTAs, and if there are still fewer CTAs than jobs every warp takes rows or half rows on its own. A CTA that
+    // merges one row after the other pays a trip to L2 and five barriers for each (10 layers with a window of 513 keys, 20
+    // CTAs for 64 rows: 180 -> 121 us a pass).
+    const bool few = !it.partial && R < FIN_JOBS;
+    const uint32_t first = ticket - (total - R), jobs = few ? 16u * it.ntok : FIN_JOBS, w = threadIdx.x >> 5;
+    if (few && R < jobs) {
+        if (R * (NT / 64u) >= jobs) { // enough warps for all half rows at once
+            const uint32_t j = first + R * (w >> 1);
+            if (j < jobs) merge_row_warp<NT, EXT, 1>(it, j & 1u, j >> 1, w & 1u);
+        } else {
+            for (uint32_t j = first + R * w; j < jobs; j += R * (NT / 32u)) merge_row_warp<NT, EXT, 2>(it, j & 1u, j >> 1, 0u);
+        }
+        return;
+    }
+    for (uint32_t j = first; j < jobs; j += R) {
+        merge_row<NT, EXT>(it, few ? 32u * (j & 1u) + (j >> 1) : j, sm, status);
         if (!sm.ok) return;
     }
 #ifdef MKV_TRACE

@@ -471,6 +471,27 @@ def test_window_and_sinks_on_an_ordinary_cache(ctx, oracle, fmt):
     cache.close()
 
 
+@pytest.mark.parametrize("fmt", FMTS)
+@pytest.mark.parametrize("ntok", [1, 3, 4])
+def test_merge_of_any_number_of_pieces(ctx, oracle, fmt, ntok):
+    """Windows of 1 ... 33 pieces of 128 keys: rows merged by warps (whole rows with the fewest CTAs, then half rows) and, from one
+    CTA a row on, by CTAs."""
+    pos = 5000
+    cache = kv.KvCache(ctx, fmt, 1, 6144)
+    kc, vc = fill_both(oracle, cache, 0, pos + ntok, 96)
+    q = synth.normal(96, synth.S_Q, 0, (ntok, 16, 256))
+    sinks = np.linspace(1.0, -1.0, 16).astype(np.float32)
+    for n in (1, 2, 3, 4, 7, 8, 9, 15, 16, 17, 24, 31, 32, 33):
+        out = torch.full((ntok + 1, 16, 256), float("nan"), device="cuda")
+        sk = sinks if n % 2 else None
+        cache.attn_verify_window(0, 128 * n - 3, None if sk is None else dev(sk), pos, dev(q), out[:ntok])
+        ctx.sync()
+        got = out.cpu().numpy()
+        assert np.isnan(got[ntok]).all()
+        assert oracle.max_rel(got[:ntok], oracle.attn_window_f64(int(fmt), kc, vc, 0, 128 * n - 3, sk, pos, q)) < WTOL[fmt], n
+    cache.close()
+
+
 def test_ring_cache_limits(ctx):
     with pytest.raises(kv.MkvError):
         kv.KvCache(ctx, kv.KvFormat.F16, 1, 8192, ring=1000)  # not a multiple of 128
