@@ -789,9 +789,17 @@ extern "C" mkv_status mkv_static_status(int device, void *stream, uint32_t *stat
 namespace mkv {
 
 // Chooses tiles_per_split so that all items together fill the SMs in one wave (one CTA per SM), and lays
-// the items out in the flattened grid. Items must have tile_begin / tile_end set. (A piece need not be a whole number
-// of the kernels' tiles: they do not fetch the part of a last tile that lies past the piece.)
-void plan_items(Ctx *ctx, VerifyItem *items, int n) {
+// the items out in the flattened grid. Items must have tile_begin / tile_end set.
+//
+// The pieces of a single item are whole numbers of the kernels' 128-key tiles (`step` units). A tile costs the same MMAs and
+// softmax whether it is full or not, and a short context's first tile is loaded while the kernel in front still runs, so
+// smaller pieces only make more CTAs to wait for and more pieces to merge. us a layer in a chain, 4 tokens, f16, pieces of
+// any number of 64-key units / of whole tiles: 1,000 tokens 12.9 / 10.9, 4,096 12.6 / 11.9, 14,000 15.2 / 14.0, 23,451 17.5 /
+// 16.3, 40,000 21.9 / 21.5, the same at 65,536; f32 (32-key units): 500 18.9 / 16.8, 14,000 24.6 / 23.9, 40,000 45.0 / 44.3.
+// A batch shares one piece length among its items, and the finer step comes closer to one wave (25 sessions of 1,701 to 4,700
+// tokens: 81 us a layer, in whole tiles 98).
+void plan_items(Ctx *ctx, mkv_fmt fmt, VerifyItem *items, int n) {
+    const uint32_t step = n == 1 ? 128u / (fmt == MKV_F16 ? TILE : TILE32) : 1u;
     uint64_t tiles = 0;
     uint32_t min_tps = 1;
     for (int i = 0; i < n; i++) {
@@ -803,7 +811,7 @@ void plan_items(Ctx *ctx, VerifyItem *items, int n) {
     const uint32_t budget = (uint32_t)ctx->sm_count;
     uint32_t tps = (uint32_t)((tiles + budget - 1) / budget);
     if (tps < min_tps) tps = min_tps;
-    for (;; tps++) {
+    for (tps = (tps + step - 1u) / step * step;; tps += step) {
         uint64_t ctas = 0;
         for (int i = 0; i < n; i++) ctas += 2ull * ((items[i].tile_end - items[i].tile_begin + tps - 1) / tps);
         if (ctas <= budget || ctas <= 2ull * (uint64_t)n) break; // one wave, or nothing left to merge
