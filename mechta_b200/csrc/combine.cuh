@@ -6,11 +6,13 @@
 // The sums run over the pieces in index order, so a result does not depend on timing.
 //
 // Scheduling. Every CTA writes its piece and publishes it: the threads that wrote it meet at a barrier, one of
-// them issues a release fence and takes a ticket from a counter in global memory. The last R = min(CTAs of the
-// item, 64) arrivals wait (bounded) until the counter shows that all pieces are there, and each merges a share of
-// the item's 64 rows (or rows of warps, see finish_item). Only CTAs that have finished their own work ever wait, and fewer of them than there are SMs,
-// so the others always make progress; the earlier arrivals leave at once, which lets the CTAs of the next launch
-// in the stream start on their SMs and load their first tiles.
+// them issues a release fence and takes a ticket from a counter in global memory. R = min(CTAs of the item, 64) arrivals wait
+// (bounded) until the counter shows that all pieces are there, and each merges a share of the item's 64 rows (or its warps do,
+// see finish_item). They are the last but FIN_LATE: the very last ones would have their teardown still to do when the others
+// can merge, the first ones would hold their SMs for longest (4 tokens over 65,536, us a layer, the last 64 / the last but 20 /
+// but 40 / the first 64: 29.0 / 28.7 / 28.65 / 29.2; over 9,001: 12.8 / 12.4 / 12.2 / 12.3). Only CTAs that have finished their
+// own work ever wait, and fewer of them than there are SMs, so the others always make progress; the rest leave at once, which
+// lets the CTAs of the next launch in the stream start on their SMs and load their first tiles.
 // (Measured against this: per-piece flags with merging CTAs that gather the pieces as they land, whole rows or
 // half rows per CTA. The CTAs that wait hold their SMs, the next launch's CTAs start later and find their first
 // tiles not yet loaded when they may begin: 3 to 4 % slower at 65,536 tokens.)
@@ -57,6 +59,7 @@ constexpr int FIN_MAX_THREADS = 512;
 constexpr long long FIN_WAIT_LIMIT = 4000000000ll; // about two seconds of SM clocks
 constexpr uint32_t FIN_JOBS = 64;                  // one job per row (kvh * 32 + row) of the item
 constexpr uint32_t FIN_COLS = 64;                  // float4 columns of a row
+constexpr uint32_t FIN_LATE = 40;                  // arrivals after the merging ones
 
 struct FinishSmem {
     float e_s[MAX_SPLITS];
@@ -337,6 +340,66 @@ __device__ __forceinline__ void merge_row_warp(const VerifyItem &it, uint32_t kv
     for (int h = 0; h < H; h++) store_row(it, tok, head, c4 + 32u * h, acc[h], 1.0f / tot, gate[h]);
 }
 
+// A row of one item by the 256 threads of a CTA of the f16 kernels (final outputs only): the same sums, without shared memory. A
+// warp takes 8 of the row's 64 float4 columns, its lanes in four groups that take every fourth piece; every load goes out at
+// once, every warp works out the maximum and the weights for itself, and the groups meet in shuffles. merge_row's five barriers
+// cost more: 4 tokens, us a layer in a chain, merge_row / this one: 4,096 tokens 11.6 / 10.9, 23,451 16.1 / 15.4, 65,536 29.5 /
+// 29.0. On the f32 kernel's 16 warps (64 bytes of a piece each) it was slower: 9,001 tokens 19.3 / 20.5.
+template <bool EXT>
+__device__ __forceinline__ void merge_row_cta(const VerifyItem &it, uint32_t kvh, uint32_t row, FinishSmem &sm) {
+    constexpr uint32_t COLS = 8, GROUPS = 4, RND = MAX_SPLITS / GROUPS;
+    const uint32_t lane = threadIdx.x & 31u, grp = lane / COLS, c4 = COLS * (threadIdx.x >> 5) + lane % COLS;
+    const uint32_t tok = row >> 3, head = 8u * kvh + (row & 7u), ns = it.nsplit;
+    const float2 *ml = reinterpret_cast<const float2 *>(it.part_ml) + (size_t)kvh * ns * 32u + row;
+    const float4 *po = reinterpret_cast<const float4 *>(it.part_o + ((size_t)kvh * ns * 32u + row) * 256u) + c4;
+    float2 y[3];
+#pragma unroll
+    for (uint32_t i = 0; i < 3u; i++) y[i] = lane + 32u * i < ns ? __ldcg(ml + (size_t)(lane + 32u * i) * 32u) : make_float2(NEG_BIG, 0.0f);
+    float4 x[RND], gate = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (uint32_t i = 0; i < RND; i++) x[i] = grp + GROUPS * i < ns ? __ldcg(po + (size_t)(grp + GROUPS * i) * 2048u) : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (it.gate && grp == 0u) gate = __ldg(reinterpret_cast<const float4 *>(it.gate + ((size_t)tok * 16u + head) * 512u + 256u) + c4);
+#ifdef MKV_TRACE
+    if (threadIdx.x == 0) asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(sm.tm[0]));
+#endif
+    float M = fmaxf(fmaxf(y[0].x, y[1].x), y[2].x);
+#pragma unroll
+    for (int sh = 16; sh > 0; sh >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, sh));
+    if (EXT && it.sinks) M = fmaxf(M, it.sinks[head]); // joins the maximum and the sum, never the output
+    float e[3], tot = 0.0f;
+#pragma unroll
+    for (uint32_t i = 0; i < 3u; i++) {
+        e[i] = lane + 32u * i < ns ? expf(y[i].x - M) : 0.0f;
+        tot += e[i] * y[i].y;
+    }
+#pragma unroll
+    for (int sh = 16; sh > 0; sh >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, sh);
+    if (EXT && it.sinks) tot += expf(it.sinks[head] - M);
+#ifdef MKV_TRACE
+    if (threadIdx.x == 0) asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(sm.tm[1]));
+#endif
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (uint32_t i = 0; i < RND; i++) { // piece grp + GROUPS * i: its weight is in lane (piece % 32), register piece / 32
+        const float w = __shfl_sync(0xffffffffu, e[GROUPS * i / 32u], (int)((grp + GROUPS * i) & 31u)); // 0 from the last piece on
+        a.x += w * x[i].x;
+        a.y += w * x[i].y;
+        a.z += w * x[i].z;
+        a.w += w * x[i].w;
+    }
+#pragma unroll
+    for (uint32_t sh = COLS; sh < 32u; sh <<= 1) {
+        a.x += __shfl_xor_sync(0xffffffffu, a.x, sh);
+        a.y += __shfl_xor_sync(0xffffffffu, a.y, sh);
+        a.z += __shfl_xor_sync(0xffffffffu, a.z, sh);
+        a.w += __shfl_xor_sync(0xffffffffu, a.w, sh);
+    }
+#ifdef MKV_TRACE
+    if (threadIdx.x == 0) asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(sm.tm[2]));
+#endif
+    if (grp == 0u) store_row(it, tok, head, c4, a, 1.0f / tot, gate);
+}
+
 // The CTA's share of the merge, given its ticket (publish_piece). Called by every thread of every CTA of an item;
 // `sm` must not alias anything still in use and nobody may have touched it since a barrier. Returns after this
 // CTA's rows (possibly none).
@@ -344,7 +407,9 @@ template <int NT, bool EXT = true>
 __device__ __forceinline__ void finish_item(const VerifyItem &it, FinishSmem &sm, uint32_t *status, uint32_t ticket) {
     const uint32_t total = 2u * it.nsplit;
     const uint32_t R = total < FIN_JOBS ? total : FIN_JOBS;
-    if (ticket < total - R) return; // not among the last R: nothing to merge
+    const uint32_t late = min(total - R, FIN_LATE);
+    if (ticket + late < total - R || ticket >= total - late) return; // too early or too late: nothing to merge
+    ticket += late;
     if (threadIdx.x == 0) {
 #ifdef MKV_TRACE
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(sm.tr[0]));
@@ -383,9 +448,14 @@ __device__ __forceinline__ void finish_item(const VerifyItem &it, FinishSmem &sm
         }
         return;
     }
-    for (uint32_t j = first; j < jobs; j += R) {
-        merge_row<NT, EXT>(it, few ? 32u * (j & 1u) + (j >> 1) : j, sm, status);
-        if (!sm.ok) return;
+    if (NT == 256 && !it.partial) { // one row a CTA at most
+        const uint32_t kvh = few ? first & 1u : first >> 5, row = few ? first >> 1 : first & 31u;
+        if (first < jobs && row < 8u * it.ntok) merge_row_cta<EXT>(it, kvh, row, sm);
+    } else {
+        for (uint32_t j = first; j < jobs; j += R) {
+            merge_row<NT, EXT>(it, few ? 32u * (j & 1u) + (j >> 1) : j, sm, status);
+            if (!sm.ok) return;
+        }
     }
 #ifdef MKV_TRACE
     __syncthreads();

@@ -423,7 +423,7 @@ verify_f16_tc_kernel(const VerifyItem *__restrict__ items, int n_items, const __
             // P^T buffer j & 1 belongs to the MMAs of tile j-2 until those have completed
             if (j > 1) ok = __all_sync(0xffffffffu, vt_wait(bar_pv_done + 8u * (j & 1u), ((j >> 1) - 1u) & 1u, sh, status)) && ok;
             tc_fence_after();
-            if (vt_bar_or(over || !ok)) {
+            if (j == 0u || vt_bar_or(over || !ok)) { // (the first tile always sets the references)
                 if (vt_bar_or(!ok)) { // a wait ran out somewhere: all 128 threads leave together
                     stopped = true;
                     break;
@@ -507,40 +507,36 @@ verify_f16_tc_kernel(const VerifyItem *__restrict__ items, int n_items, const __
 
         // ---------------- the piece's partial: [m, l] per row and O[32][256] ----------------
         if (!stopped) {
-            bool ok = true;
-            if (nts > 0) ok = __all_sync(0xffffffffu, vt_wait(bar_pv_done + 8u * ((nts - 1u) & 1u), ((nts - 1u) >> 1) & 1u, sh, status));
-            tc_fence_after();
             const size_t piece = (size_t)kvh * it.nsplit + split;
             float mrow = VT_UNSET; // -(reference maximum) of row `lane`
 #pragma unroll
             for (int r = 0; r < 32; r++)
                 if (lane == (uint32_t)r) mrow = negm[r];
             float *red = red_base + 128u * (red_turn & 1u);
-            red[lane * 4u + q4] = vt_transpose_reduce<false>(lpart, lane);
+            red[lane * 4u + q4] = vt_transpose_reduce<false>(lpart, lane); // while the last product runs
             vt_bar_sync();
             if (q4 == 0) {
                 const float4 x = *reinterpret_cast<const float4 *>(red + 4 * lane);
                 const float m = mrow < 0.5f * VT_UNSET ? -mrow * 0.6931471805599453f : NEG_BIG; // back to natural units
                 reinterpret_cast<float2 *>(it.part_ml)[piece * 32u + lane] = make_float2(m, (x.x + x.y) + (x.z + x.w));
             }
+            bool ok = true;
+            if (nts > 0) ok = __all_sync(0xffffffffu, vt_wait(bar_pv_done + 8u * ((nts - 1u) & 1u), ((nts - 1u) >> 1) & 1u, sh, status));
+            tc_fence_after();
             float *po = it.part_o + piece * 32u * 256u;
+            uint32_t oc[2][32];
+            if (nts > 0 && ok) {
+                tmem_ld32(tmem + lane_addr + VT_COL_O, oc[0]);
+                tmem_ld32(tmem + lane_addr + VT_COL_O + 32u, oc[1]);
+                tmem_wait_ld();
+            } else {
 #pragma unroll
-            for (uint32_t mh = 0; mh < 2u; mh++) {
-                uint32_t oc[32];
-                if (nts > 0 && ok) {
-                    tmem_ld32(tmem + lane_addr + VT_COL_O + 32u * mh, oc);
-                    tmem_wait_ld();
-                } else {
-#pragma unroll
-                    for (int r = 0; r < 32; r++) oc[r] = 0u;
-                }
-#pragma unroll
-#ifndef VT_X_NOSTORE
-                for (int r = 0; r < 32; r++) po[(size_t)r * 256u + 128u * mh + klane] = __uint_as_float(oc[r]);
-#else
-                if (oc[0] == 0x12345678u && oc[31] == 0x9abcdef0u) po[klane] = 1.0f; // timing only: keeps the loads alive
-#endif
+                for (int r = 0; r < 32; r++) oc[0][r] = oc[1][r] = 0u;
             }
+#pragma unroll
+            for (uint32_t mh = 0; mh < 2u; mh++)
+#pragma unroll
+                for (int r = 0; r < 32; r++) po[(size_t)r * 256u + 128u * mh + klane] = __uint_as_float(oc[mh][r]);
         }
         // The piece is published by the threads that wrote it, before the CTA's teardown: what follows the last piece
         // of a launch is the critical path of the next one. (After a wait that ran out the piece is not valid; it is
@@ -556,7 +552,7 @@ verify_f16_tc_kernel(const VerifyItem *__restrict__ items, int n_items, const __
         // a wait ran out somewhere: give copies already issued into this CTA's shared memory a bounded time to land
         for (int s = 0; s < VT_NSLOT; s++) mbar_wait_bounded(bar_full + 8u * s, 0, 200000000ll);
     }
-    __syncthreads();
+    if (sh->abort) __syncthreads();
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem, VT_COLS);
