@@ -56,6 +56,7 @@ constexpr long long PS_WAIT_LIMIT = 2000000000ll;
 constexpr float PS_LOG2E = 1.4426950408889634f;
 constexpr float PS_C2 = SCALE * PS_LOG2E;              // scores to base-2 exponents
 constexpr float PS_LAZY2 = 8.0f * PS_LOG2E;
+constexpr PfCost PS_COST = {1.4f, 0.6f, 0.023f};       // a tile takes about 5.6 us
 static_assert(PS_SMEM <= 232448, "shared memory of prefill_f32_tc_kernel");
 
 struct PsShared {
@@ -482,10 +483,11 @@ prefill_f32_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
             } else {
                 // a part of an item: its partial goes to scratch memory for the merge kernel
                 float *ps = scratch + pf_slot(pair, sg.piece, cta) * PF_PART;
-                if (half == 0u) *reinterpret_cast<float2 *>(ps + 128u * 256u + 2u * row) = make_float2(m_ref, l_all);
+                const bool real = tok0 + (row & 15u) < plan.ntok; // (rows beyond the block are neither written nor read)
+                if (half == 0u && real) *reinterpret_cast<float2 *>(ps + 128u * 256u + 2u * row) = make_float2(m_ref, l_all);
 #pragma unroll
                 for (uint32_t c = 0; c < 32u; c++)
-                    *reinterpret_cast<float4 *>(ps + ((size_t)(32u * half + c) * 128u + row) * 4u) =
+                    if (real) *reinterpret_cast<float4 *>(ps + ((size_t)(32u * half + c) * 128u + row) * 4u) =
                         make_float4(acc[4u * c], acc[4u * c + 1u], acc[4u * c + 2u], acc[4u * c + 3u]);
             }
             pair_bar_sync(1u + q4); // red[] is free for the next segment
@@ -515,12 +517,12 @@ mkv_status prefill_f32_tc_setup_device() {
 }
 
 mkv_status launch_prefill_f32_tc(Ctx *ctx, Cache *c, int layer, uint32_t first_pos, uint32_t pos0, uint32_t ntok, const float *q, float *out) {
-    const PfPlan plan = pf_plan(ctx, first_pos, pos0, ntok);
+    const PfPlan plan = pf_plan(ctx, PS_COST, first_pos, pos0, ntok);
     mkv_status st = prefill_scratch(ctx);
     if (st != MKV_OK) return st;
     const CUtensorMap &km = c->maps_host[2 * (c->n_layers + layer)], &vm = c->maps_host[2 * (c->n_layers + layer) + 1];
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2u * pf_pairs(plan));
+    cfg.gridDim = dim3(2u * plan.pairs);
     cfg.blockDim = dim3(PS_THREADS);
     cfg.dynamicSmemBytes = PS_SMEM;
     cfg.stream = ctx->stream;

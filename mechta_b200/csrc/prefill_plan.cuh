@@ -6,18 +6,20 @@
 namespace mkv {
 
 constexpr uint32_t PF_KEYS = 128;   // keys per tile
-constexpr uint32_t PF_MIN_LEN = 2;  // tiles a pair takes at least: a shorter range costs more in partials than it saves
 // One partial of a CTA: O as [64 chunks of 4 dims][128 rows][4] (a warp's rows store and load 512 contiguous bytes), then
 // [128 rows][m, l]
 constexpr size_t PF_PART = 128u * 256u + 128u * 2u;
 
 // The work of one launch. Items are numbered longest first: item i = (group of 32 tokens ngroups - 1 - i / 2, KV head i % 2);
-// its tiles are the 128-key tiles from first_pos / 128 up to the last key its last token sees. Pair p takes the tiles
-// [p * len, (p + 1) * len) of all items laid end to end.
+// its tiles are the 128-key tiles from first_pos / 128 up to the last key its last token sees. Pairs of CTAs take
+//   per = 1: whole items, item after item to and fro over the pairs;
+//   per > 1: one of `per` equal parts of an item each;
+//   per = 0: the tiles [p * len, (p + 1) * len) of all items laid end to end.
 struct PfPlan {
     uint32_t first_pos, pos0, ntok;
     uint32_t ngroups, nitems, t0;
-    uint32_t total, len;
+    uint32_t per, pairs;
+    uint32_t total, len; // per = 0
     __host__ __device__ uint32_t group_of(uint32_t item) const { return ngroups - 1u - (item >> 1); }
     __host__ __device__ uint32_t item_end(uint32_t item) const { // the token after the item's last one
         const uint32_t e = group_of(item) * 32u + 32u;
@@ -26,6 +28,7 @@ struct PfPlan {
     __host__ __device__ uint32_t tiles_of(uint32_t item) const {
         return (pos0 + item_end(item) + PF_KEYS - 1u) / PF_KEYS - t0;
     }
+    __host__ __device__ uint32_t part_len(uint32_t n) const { return (n + per - 1u) / per; } // per > 0: tiles of a part of an item of n tiles
 };
 struct PfSegment {
     uint32_t item, a, b;     // tiles [a, b) of the item
@@ -34,12 +37,21 @@ struct PfSegment {
 // Walks the segments of one pair.
 struct PfWalk {
     const PfPlan &p;
-    uint32_t pair, lo, hi, item, base;
+    uint32_t pair, lo, hi, item, base; // per > 0: base = rounds over the pairs so far
     __device__ __forceinline__ PfWalk(const PfPlan &plan, uint32_t pair_) : p(plan), pair(pair_), item(0), base(0) {
         lo = min(pair * p.len, p.total);
         hi = min(lo + p.len, p.total);
     }
     __device__ __forceinline__ bool next(PfSegment &s) {
+        if (p.per > 0u) {
+            const uint32_t u = base * p.pairs + ((base & 1u) ? p.pairs - 1u - pair : pair);
+            base++;
+            if (u >= p.nitems * p.per) return false;
+            const uint32_t it = u / p.per, piece = u % p.per, n = p.tiles_of(it), l = p.part_len(n);
+            if (piece * l >= n) return false; // (per > 1, where a pair has one part: an item of so few tiles has fewer parts)
+            s = {it, piece * l, min(piece * l + l, n), piece, (n + l - 1u) / l};
+            return true;
+        }
         while (item < p.nitems && base < hi) {
             const uint32_t n = p.tiles_of(item), a = max(base, lo), b = min(base + n, hi);
             if (b > a) {
@@ -60,8 +72,12 @@ __host__ __device__ inline size_t pf_slot(uint32_t pair, uint32_t piece, uint32_
     return ((size_t)pair * 2u + (piece == 0u ? 1u : 0u)) * 2u + cta;
 }
 
-PfPlan pf_plan(Ctx *ctx, uint32_t first_pos, uint32_t pos0, uint32_t ntok);
-inline uint32_t pf_pairs(const PfPlan &p) { return (p.total + p.len - 1u) / p.len; }
+// What parts cost a kernel, in units of its time for a tile: a segment (queries, pipeline, outputs or partial), the launch of the
+// merge, and a part's way through memory.
+struct PfCost {
+    float segment, merge, part;
+};
+PfPlan pf_plan(Ctx *ctx, const PfCost &cost, uint32_t first_pos, uint32_t pos0, uint32_t ntok);
 // Scratch of the split items: two partials per CTA, allocated with the context's first prefill launch and kept until the
 // context goes.
 mkv_status prefill_scratch(Ctx *ctx);

@@ -15,12 +15,12 @@
 // in a burst run at 1,345). The waits use mbarrier.try_wait at its default scope: with .acquire.cluster, which costs a cache
 // invalidation each time, the same kernel took 1,032 us a layer instead of 843.
 //
-// Scheduling. The grid is one pair of CTAs per two SMs, and the 128-key tiles of all items, laid end to end (longest items
-// first), are cut into equal ranges, one per pair. A pair walks its range segment by segment; a segment that covers its whole
-// item writes the output, a part of an item writes its un-normalised partial (reference maximum, sum, O) to scratch memory,
-// and a second small kernel merges the parts in index order over the whole chip (the reference splits long prefills over
-// chunks and merges with attn_fd_combine in the same way, M/engine.rs:1219-1225). 200 tokens over 9,001: 256 -> 52 us a layer
-// (one CTA per split item used to merge it alone, with uncoalesced loads).
+// Scheduling. The grid is at most one pair of CTAs per two SMs; pf_plan decides what each pair takes: whole items, equal parts
+// of items, or equal ranges of the tiles of all items laid end to end (prefill_plan.cuh). A pair walks its work segment by
+// segment; a segment that covers its whole item writes the output, a part of an item writes its un-normalised partial
+// (reference maximum, sum, O) to scratch memory, and a second small kernel merges the parts in index order over the whole chip
+// (the reference splits long prefills over chunks and merges with attn_fd_combine in the same way, M/engine.rs:1219-1225). 200
+// tokens over 9,001: 256 -> 40 us a layer (one CTA per split item used to merge it alone, with uncoalesced loads).
 //
 // Roles (320 threads): warp 0 = TMA producer, warp 1 = MMA issuer (one thread, of the pair's first CTA only) and TMEM owner,
 // warps 2..9 = softmax, two threads per row (64 of a tile's 128 keys each). Per tile: S = Q K^T (16 MMAs, A = Q from tensor
@@ -58,6 +58,7 @@ constexpr long long TC_WAIT_LIMIT = 2000000000ll;
 constexpr float TC_LOG2E = 1.4426950408889634f;
 constexpr float TC_LAZY2 = 8.0f * TC_LOG2E;
 constexpr float TC_C2 = SCALE * TC_LOG2E;              // scores to base-2 exponents
+constexpr PfCost TC_COST = {2.8f, 1.7f, 0.075f};     // a tile takes about 1.75 us
 static_assert(TC_SMEM <= 232448, "shared memory of prefill_f16_tc_kernel");
 
 struct TcShared {
@@ -410,7 +411,8 @@ prefill_f16_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
             } else {
                 // a part of an item: its partial goes to scratch memory for the merge kernel
                 float *ps = scratch + pf_slot(pair, sg.piece, cta) * PF_PART;
-                if (half == 0u) *reinterpret_cast<float2 *>(ps + 128u * 256u + 2u * row) = make_float2(m_ref, l_all);
+                const bool real = tok0 + (row & 15u) < plan.ntok; // (rows beyond the block are neither written nor read)
+                if (half == 0u && real) *reinterpret_cast<float2 *>(ps + 128u * 256u + 2u * row) = make_float2(m_ref, l_all);
 #pragma unroll 1
                 for (uint32_t c0 = 0; c0 < 128u; c0 += 32u) {
                     uint32_t orow[32];
@@ -418,7 +420,7 @@ prefill_f16_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
                     tmem_wait_ld();
 #pragma unroll
                     for (int c = 0; c < 32; c += 4)
-                        *reinterpret_cast<uint4 *>(ps + ((size_t)((128u * half + c0 + c) >> 2) * 128u + row) * 4u) =
+                        if (real) *reinterpret_cast<uint4 *>(ps + ((size_t)((128u * half + c0 + c) >> 2) * 128u + row) * 4u) =
                             make_uint4(orow[c], orow[c + 1], orow[c + 2], orow[c + 3]);
                 }
             }
@@ -454,11 +456,20 @@ prefill_merge_kernel(const __grid_constant__ PfPlan plan, const float *__restric
     pdl_launch_dependents();
     const uint32_t item = blockIdx.y, cta = blockIdx.x >> 5, q4 = (blockIdx.x >> 3) & 3u, eighth = blockIdx.x & 7u;
     const uint32_t lane = threadIdx.x & 31u, grp = threadIdx.x >> 6, ch = (threadIdx.x >> 5) & 1u, row = 32u * q4 + lane;
-    uint32_t base = 0;
-    for (uint32_t i = 0; i < item; i++) base += plan.tiles_of(i);
-    const uint32_t n = plan.tiles_of(item), p0 = base / plan.len, np = (base + n - 1u) / plan.len - p0 + 1u;
+    const uint32_t n = plan.tiles_of(item);
+    uint32_t p0, np; // the pair of the item's first part, the number of its parts
+    if (plan.per > 0u) {
+        p0 = item * plan.per;
+        np = (n + plan.part_len(n) - 1u) / plan.part_len(n);
+    } else {
+        uint32_t base = 0;
+        for (uint32_t i = 0; i < item; i++) base += plan.tiles_of(i);
+        p0 = base / plan.len;
+        np = (base + n - 1u) / plan.len - p0 + 1u;
+    }
     const uint32_t tok0 = plan.group_of(item) * 32u + 16u * cta;
     if (np == 1u || tok0 >= plan.ntok) return; // written by the attention kernel, or padding
+    const bool real = tok0 + (row & 15u) < plan.ntok;
     pdl_wait();
     float M = NEG_BIG, l = 0.0f;
     float4 acc[4];
@@ -471,10 +482,10 @@ prefill_merge_kernel(const __grid_constant__ PfPlan plan, const float *__restric
         for (uint32_t k = 0; k < 4u; k++) {
             const uint32_t s = s0 + 4u * k;
             const float *ps = scratch + pf_slot(p0 + min(s, np - 1u), s, cta) * PF_PART; // (s > 0 from the second part on)
-            ml[k] = s < np ? __ldcg(reinterpret_cast<const float2 *>(ps + 128u * 256u + 2u * row)) : make_float2(NEG_BIG, 0.0f);
+            ml[k] = s < np && real ? __ldcg(reinterpret_cast<const float2 *>(ps + 128u * 256u + 2u * row)) : make_float2(NEG_BIG, 0.0f);
 #pragma unroll
             for (uint32_t i = 0; i < 4u; i++)
-                v[k][i] = s < np ? __ldcg(reinterpret_cast<const float4 *>(ps + ((size_t)(8u * eighth + 4u * ch + i) * 128u + row) * 4u))
+                v[k][i] = s < np && real ? __ldcg(reinterpret_cast<const float4 *>(ps + ((size_t)(8u * eighth + 4u * ch + i) * 128u + row) * 4u))
                                  : make_float4(0.f, 0.f, 0.f, 0.f);
         }
         const float mx = fmaxf(fmaxf(ml[0].x, ml[1].x), fmaxf(ml[2].x, ml[3].x));
@@ -539,7 +550,12 @@ mkv_status prefill_scratch(Ctx *ctx) {
     return MKV_OK;
 }
 
-PfPlan pf_plan(Ctx *ctx, uint32_t first_pos, uint32_t pos0, uint32_t ntok) {
+// Chooses the way of the three that the cost model expects to be the fastest. Whole items need no merge but leave pairs idle
+// when there are few; equal parts are one segment a pair; the end-to-end cut is even for any number of items but gives a pair
+// several segments. Measured against the
+// end-to-end cut alone (us a layer): 1,226 tokens over 91 77 -> 29 and 1,121 over 1,779 96 -> 51 (whole items), 200 over 9,001 45.3
+// -> 40.2 (five parts an item), 32 over 9,001 24.6 -> 20.1, 5 over 16 18.5 -> 11.6; 2,048 over 32,768 is still cut end to end.
+PfPlan pf_plan(Ctx *ctx, const PfCost &cost, uint32_t first_pos, uint32_t pos0, uint32_t ntok) {
     PfPlan plan;
     plan.first_pos = first_pos; plan.pos0 = pos0; plan.ntok = ntok;
     plan.ngroups = (ntok + 31u) / 32u;
@@ -547,18 +563,49 @@ PfPlan pf_plan(Ctx *ctx, uint32_t first_pos, uint32_t pos0, uint32_t ntok) {
     plan.t0 = first_pos / PF_KEYS;
     plan.total = 0;
     for (uint32_t i = 0; i < plan.nitems; i += 2u) plan.total += 2u * plan.tiles_of(i);
-    const uint32_t npairs = (uint32_t)ctx->sm_count / 2u;
-    plan.len = std::max((plan.total + npairs - 1u) / npairs, PF_MIN_LEN);
+    const uint32_t npairs = (uint32_t)ctx->sm_count / 2u, n = plan.nitems, longest = plan.tiles_of(0), shortest = plan.tiles_of(n - 1u);
+    plan.len = (plan.total + npairs - 1u) / npairs;
+    // end to end
+    float best = (float)plan.len + (1.0f + (float)plan.len / (float)shortest) * cost.segment + cost.merge + cost.part * (float)(npairs + n);
+    plan.per = 0;
+    plan.pairs = (plan.total + plan.len - 1u) / plan.len;
+    { // whole items: the pair that gets the most
+        const uint32_t rounds = (n + npairs - 1u) / npairs;
+        uint32_t most = longest;
+        for (uint32_t p = 0; rounds > 1u && p < npairs; p++) {
+            uint32_t t = 0;
+            for (uint32_t k = 0; k < rounds; k++) {
+                const uint32_t u = k * npairs + ((k & 1u) ? npairs - 1u - p : p);
+                if (u < n) t += plan.tiles_of(u);
+            }
+            most = std::max(most, t);
+        }
+        const float t = (float)most + (float)rounds * cost.segment;
+        if (t <= best) {
+            best = t;
+            plan.per = 1;
+            plan.pairs = std::min(n, npairs);
+        }
+    }
+    for (uint32_t per = 2; per * n <= npairs && per <= longest; per++) { // equal parts
+        const float t = (float)((longest + per - 1u) / per) + cost.segment + cost.merge + cost.part * (float)(per * n);
+        if (t < best) {
+            best = t;
+            plan.per = per;
+            plan.pairs = per * n;
+        }
+    }
     return plan;
 }
 
 mkv_status launch_prefill_merge(Ctx *ctx, const PfPlan &plan, float *out) {
     bool split = false;
-    for (uint32_t i = 0, base = 0; i < plan.nitems && !split; i++) {
+    for (uint32_t i = 0, base = 0; plan.per == 0u && i < plan.nitems && !split; i++) {
         const uint32_t n = plan.tiles_of(i);
         split = base / plan.len != (base + n - 1u) / plan.len;
         base += n;
     }
+    if (plan.per > 1u) split = plan.part_len(plan.tiles_of(0)) < plan.tiles_of(0);
     if (!split) return MKV_OK;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(64u, plan.nitems);
@@ -581,12 +628,12 @@ mkv_status launch_prefill_f16_tc(Ctx *ctx, Cache *c, int layer, uint32_t first_p
 #else
     const uint32_t phase = 0u;
 #endif
-    const PfPlan plan = pf_plan(ctx, first_pos, pos0, ntok);
+    const PfPlan plan = pf_plan(ctx, TC_COST, first_pos, pos0, ntok);
     mkv_status st = prefill_scratch(ctx);
     if (st != MKV_OK) return st;
     const CUtensorMap &km = c->maps_host[2 * (c->n_layers + layer)], &vm = c->maps_host[2 * (c->n_layers + layer) + 1];
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2u * pf_pairs(plan));
+    cfg.gridDim = dim3(2u * plan.pairs);
     cfg.blockDim = dim3(TC_THREADS);
     cfg.dynamicSmemBytes = TC_SMEM;
     cfg.stream = ctx->stream;
