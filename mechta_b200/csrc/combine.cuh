@@ -166,9 +166,8 @@ __device__ __forceinline__ void store_row(const VerifyItem &it, uint32_t tok, ui
     }
 }
 
-// One row (kvh * 32 + row) of one item, by all NT threads of the CTA; all pieces are in global memory.
-// EXT = false compiles the sink handling out (the kernels of the plain path are instantiated without it).
-template <int NT, bool EXT>
+// One row (kvh * 32 + row) of a shard's record, by all NT threads of the CTA; all pieces are in global memory.
+template <int NT>
 __device__ __forceinline__ void merge_row(const VerifyItem &it, uint32_t r, FinishSmem &sm, uint32_t *status) {
     constexpr int GROUPS = NT / FIN_COLS;
     constexpr int NW = NT / 32;
@@ -176,7 +175,7 @@ __device__ __forceinline__ void merge_row(const VerifyItem &it, uint32_t r, Fini
     const uint32_t kvh = r >> 5, row = r & 31u, tok = row >> 3, head = 8u * kvh + (row & 7u);
     const uint32_t tid = threadIdx.x;
     if (tok >= it.ntok) {
-        if (it.partial && !it.push && tid < 258u) // rows of tokens beyond the step: the empty record
+        if (!it.push && tid < 258u) // rows of tokens beyond the step: the empty record
             it.out[(size_t)(tok * 16u + head) * REC + tid] = tid == 0 ? NEG_BIG : 0.0f;
         return;
     }
@@ -186,10 +185,6 @@ __device__ __forceinline__ void merge_row(const VerifyItem &it, uint32_t r, Fini
     const float4 *po = reinterpret_cast<const float4 *>(it.part_o + ((size_t)kvh * ns * 32u + row) * 256u) + c4;
     float4 x[RND];
     float m = NEG_BIG, l = 0.0f;
-    // the head's gate values, if any, with the first loads: at the end of the row they would be one more round trip
-    float4 gate = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (!it.partial && it.gate && tid < FIN_COLS)
-        gate = __ldg(reinterpret_cast<const float4 *>(it.gate + ((size_t)tok * 16u + head) * 512u + 256u + 4 * tid));
     if (tid < ns) { // (m, l) first: the maximum is needed before anything can be summed
         const float2 y = __ldcg(ml + (size_t)tid * 32u);
         m = y.x;
@@ -213,9 +208,7 @@ __device__ __forceinline__ void merge_row(const VerifyItem &it, uint32_t r, Fini
         float y = tid < NW ? sm.red[tid] : NEG_BIG;
 #pragma unroll
         for (int sh = 16; sh > 0; sh >>= 1) y = fmaxf(y, __shfl_xor_sync(0xffffffffu, y, sh));
-        // a sink logit of the row's head joins the maximum and the sum, never the output (ggml's soft_max with sinks,
-        // W/flint_attn.wgsl:243-255)
-        if (tid == 0) sm.M = (EXT && it.sinks && !it.partial) ? fmaxf(y, it.sinks[head]) : y;
+        if (tid == 0) sm.M = y;
     }
     __syncthreads();
     M = sm.M;
@@ -233,7 +226,7 @@ __device__ __forceinline__ void merge_row(const VerifyItem &it, uint32_t r, Fini
         float y = tid < NW ? sm.red[tid] : 0.0f;
 #pragma unroll
         for (int sh = 16; sh > 0; sh >>= 1) y += __shfl_xor_sync(0xffffffffu, y, sh);
-        if (tid == 0) sm.tot = (EXT && it.sinks && !it.partial) ? y + expf(it.sinks[head] - sm.M) : y;
+        if (tid == 0) sm.tot = y;
     }
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
@@ -258,33 +251,29 @@ __device__ __forceinline__ void merge_row(const VerifyItem &it, uint32_t r, Fini
             a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
         }
         const float tot = sm.tot;
-        if (it.partial) {
-            if (it.push) { // the row goes to every rank's mailbox: plain peer stores over NVLink (no multicast), one word per value
-                const PushInfo &P = *it.push;
-                for (uint32_t dd = 0; dd < P.world; dd++) {
-                    unsigned long long *rec = P.slot[it.push_epoch & 1u][dd];
-                    if (!rec) continue; // a rank that never joined the exchange
-                    rec += (size_t)(tok * 16u + head) * REC;
-                    ptx::st_relaxed_sys_u64(rec + 2 + 4 * tid, exch_word(a.x, it.push_epoch));
-                    ptx::st_relaxed_sys_u64(rec + 3 + 4 * tid, exch_word(a.y, it.push_epoch));
-                    ptx::st_relaxed_sys_u64(rec + 4 + 4 * tid, exch_word(a.z, it.push_epoch));
-                    ptx::st_relaxed_sys_u64(rec + 5 + 4 * tid, exch_word(a.w, it.push_epoch));
-                    if (tid == 0) {
-                        ptx::st_relaxed_sys_u64(rec, exch_word(M, it.push_epoch));
-                        ptx::st_relaxed_sys_u64(rec + 1, exch_word(tot, it.push_epoch));
-                    }
+        if (it.push) { // the row goes to every rank's mailbox: plain peer stores over NVLink (no multicast), one word per value
+            const PushInfo &P = *it.push;
+            for (uint32_t dd = 0; dd < P.world; dd++) {
+                unsigned long long *rec = P.slot[it.push_epoch & 1u][dd];
+                if (!rec) continue; // a rank that never joined the exchange
+                rec += (size_t)(tok * 16u + head) * REC;
+                ptx::st_relaxed_sys_u64(rec + 2 + 4 * tid, exch_word(a.x, it.push_epoch));
+                ptx::st_relaxed_sys_u64(rec + 3 + 4 * tid, exch_word(a.y, it.push_epoch));
+                ptx::st_relaxed_sys_u64(rec + 4 + 4 * tid, exch_word(a.z, it.push_epoch));
+                ptx::st_relaxed_sys_u64(rec + 5 + 4 * tid, exch_word(a.w, it.push_epoch));
+                if (tid == 0) {
+                    ptx::st_relaxed_sys_u64(rec, exch_word(M, it.push_epoch));
+                    ptx::st_relaxed_sys_u64(rec + 1, exch_word(tot, it.push_epoch));
                 }
-            } else { // the un-normalised record itself (records are 8-byte aligned only)
-                float *rec = it.out + (size_t)(tok * 16u + head) * REC;
-                *reinterpret_cast<float2 *>(rec + 2 + 4 * tid) = make_float2(a.x, a.y);
-                *reinterpret_cast<float2 *>(rec + 4 + 4 * tid) = make_float2(a.z, a.w);
-                if (tid == 0) *reinterpret_cast<float2 *>(rec) = make_float2(M, tot);
             }
-        } else {
-            store_row(it, tok, head, tid, a, 1.0f / tot, gate);
+        } else { // the un-normalised record itself (records are 8-byte aligned only)
+            float *rec = it.out + (size_t)(tok * 16u + head) * REC;
+            *reinterpret_cast<float2 *>(rec + 2 + 4 * tid) = make_float2(a.x, a.y);
+            *reinterpret_cast<float2 *>(rec + 4 + 4 * tid) = make_float2(a.z, a.w);
+            if (tid == 0) *reinterpret_cast<float2 *>(rec) = make_float2(M, tot);
         }
     }
-    if (it.partial && it.push && !exchange_row<NT>(*it.push, it.push_epoch, tok * 16u + head, it.out, status, sm.red)) {
+    if (it.push && !exchange_row<NT>(*it.push, it.push_epoch, tok * 16u + head, it.out, status, sm.red)) {
         if (tid == 0) sm.ok = 0u; // a rank never delivered: the CTA's other rows would only wait as long again
         __syncthreads();
     }
@@ -340,15 +329,17 @@ __device__ __forceinline__ void merge_row_warp(const VerifyItem &it, uint32_t kv
     for (int h = 0; h < H; h++) store_row(it, tok, head, c4 + 32u * h, acc[h], 1.0f / tot, gate[h]);
 }
 
-// A row of one item by the 256 threads of a CTA of the f16 kernels (final outputs only): the same sums, without shared memory. A
-// warp takes 8 of the row's 64 float4 columns, its lanes in four groups that take every fourth piece; every load goes out at
-// once, every warp works out the maximum and the weights for itself, and the groups meet in shuffles. merge_row's five barriers
-// cost more: 4 tokens, us a layer in a chain, merge_row / this one: 4,096 tokens 11.6 / 10.9, 23,451 16.1 / 15.4, 65,536 29.5 /
-// 29.0. On the f32 kernel's 16 warps (64 bytes of a piece each) it was slower: 9,001 tokens 19.3 / 20.5.
-template <bool EXT>
+// A row of one item by the threads of a CTA (final outputs only): the same sums with no barrier (256 threads) or one (512). A warp
+// takes 8 of the row's 64 float4 columns, its lanes in four groups that take every fourth piece (of 16 warps, the second eight
+// take every other one of these); every load goes out at once, every warp works out the maximum and the weights for itself, and
+// the groups meet in shuffles. merge_row's five barriers cost more: 4 tokens on the f16 cache, us a layer in a chain, merge_row /
+// this one: 4,096 tokens 11.6 / 10.9, 23,451 16.1 / 15.4, 65,536 29.5 / 29.0; f32 cache: 4,096 18.1 / 17.4, 65,536 58.1 / 57.9
+// (with the row sums reduced while the last products run).
+template <int NT, bool EXT>
 __device__ __forceinline__ void merge_row_cta(const VerifyItem &it, uint32_t kvh, uint32_t row, FinishSmem &sm) {
-    constexpr uint32_t COLS = 8, GROUPS = 4, RND = MAX_SPLITS / GROUPS;
-    const uint32_t lane = threadIdx.x & 31u, grp = lane / COLS, c4 = COLS * (threadIdx.x >> 5) + lane % COLS;
+    constexpr uint32_t COLS = 8, GROUPS = NT / 64, RND = MAX_SPLITS / GROUPS;
+    static_assert(MAX_SPLITS <= 96 && MAX_SPLITS % GROUPS == 0, "a lane looks at three pieces' maxima");
+    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5, grp = lane / COLS + 4u * (w >> 3), c4 = COLS * (w & 7u) + lane % COLS;
     const uint32_t tok = row >> 3, head = 8u * kvh + (row & 7u), ns = it.nsplit;
     const float2 *ml = reinterpret_cast<const float2 *>(it.part_ml) + (size_t)kvh * ns * 32u + row;
     const float4 *po = reinterpret_cast<const float4 *>(it.part_o + ((size_t)kvh * ns * 32u + row) * 256u) + c4;
@@ -381,11 +372,11 @@ __device__ __forceinline__ void merge_row_cta(const VerifyItem &it, uint32_t kvh
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (uint32_t i = 0; i < RND; i++) { // piece grp + GROUPS * i: its weight is in lane (piece % 32), register piece / 32
-        const float w = __shfl_sync(0xffffffffu, e[GROUPS * i / 32u], (int)((grp + GROUPS * i) & 31u)); // 0 from the last piece on
-        a.x += w * x[i].x;
-        a.y += w * x[i].y;
-        a.z += w * x[i].z;
-        a.w += w * x[i].w;
+        const float f = __shfl_sync(0xffffffffu, e[GROUPS * i / 32u], (int)((grp + GROUPS * i) & 31u)); // 0 from the last piece on
+        a.x += f * x[i].x;
+        a.y += f * x[i].y;
+        a.z += f * x[i].z;
+        a.w += f * x[i].w;
     }
 #pragma unroll
     for (uint32_t sh = COLS; sh < 32u; sh <<= 1) {
@@ -393,6 +384,14 @@ __device__ __forceinline__ void merge_row_cta(const VerifyItem &it, uint32_t kvh
         a.y += __shfl_xor_sync(0xffffffffu, a.y, sh);
         a.z += __shfl_xor_sync(0xffffffffu, a.z, sh);
         a.w += __shfl_xor_sync(0xffffffffu, a.w, sh);
+    }
+    if constexpr (NT > 256) {
+        if (grp == 4u) sm.part[0][c4] = a;
+        __syncthreads();
+        if (grp == 0u) {
+            const float4 b = sm.part[0][c4];
+            a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+        }
     }
 #ifdef MKV_TRACE
     if (threadIdx.x == 0) asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(sm.tm[2]));
@@ -448,12 +447,12 @@ __device__ __forceinline__ void finish_item(const VerifyItem &it, FinishSmem &sm
         }
         return;
     }
-    if (NT == 256 && !it.partial) { // one row a CTA at most
+    if (!it.partial) { // one row a CTA at most
         const uint32_t kvh = few ? first & 1u : first >> 5, row = few ? first >> 1 : first & 31u;
-        if (first < jobs && row < 8u * it.ntok) merge_row_cta<EXT>(it, kvh, row, sm);
+        if (first < jobs && row < 8u * it.ntok) merge_row_cta<NT, EXT>(it, kvh, row, sm);
     } else {
         for (uint32_t j = first; j < jobs; j += R) {
-            merge_row<NT, EXT>(it, few ? 32u * (j & 1u) + (j >> 1) : j, sm, status);
+            merge_row<NT>(it, j, sm, status);
             if (!sm.ok) return;
         }
     }

@@ -534,7 +534,7 @@ verify_f32_tc_kernel(const VerifyItem *__restrict__ items, int n_items, const __
                             t[4 * q + 3] + n4.w > FT_LAZY2;
                 }
             }
-            if (ft_bar_or(over || !ok)) {
+            if (j == 0u || ft_bar_or(over || !ok)) { // (the first tile always sets the references)
                 if (ft_bar_or(!ok)) { // a wait ran out somewhere: all 128 threads leave together
                     stopped = true;
                     break;
@@ -627,15 +627,9 @@ verify_f32_tc_kernel(const VerifyItem *__restrict__ items, int n_items, const __
         }
         // ---------------- the piece's partial: [m, l] per row and O[32][256] ----------------
         if (!stopped) {
-            bool ok = true;
-            while (folded < nt && ok) {
-                ok = fold(folded);
-                folded++;
-            }
-            FT_STAMP(tid == FT_SOFTMAX_TID0, FP_T_FOLDED);
             const size_t piece = (size_t)kvh * it.nsplit + split;
             float *red = red_base + 128u * (red_turn & 1u);
-            red[lane * 4u + w4] = ft_transpose_reduce<false>(lpart, lane);
+            red[lane * 4u + w4] = ft_transpose_reduce<false>(lpart, lane); // while the last products run
             ft_bar_sync();
             if (w4 == 0) {
                 const float4 x = *reinterpret_cast<const float4 *>(red + 4 * lane);
@@ -643,6 +637,12 @@ verify_f32_tc_kernel(const VerifyItem *__restrict__ items, int n_items, const __
                 const float m = mrow < 0.5f * FT_UNSET ? -mrow * 0.6931471805599453f : NEG_BIG; // back to natural units
                 reinterpret_cast<float2 *>(it.part_ml)[piece * 32u + lane] = make_float2(m, (x.x + x.y) + (x.z + x.w));
             }
+            bool ok = true;
+            while (folded < nt && ok) {
+                ok = fold(folded);
+                folded++;
+            }
+            FT_STAMP(tid == FT_SOFTMAX_TID0, FP_T_FOLDED);
             float *po = it.part_o + piece * 32u * 256u + my_dim;
 #pragma unroll
             for (int p = 0; p < 4; p++)
