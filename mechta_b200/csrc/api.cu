@@ -1100,12 +1100,13 @@ mkv_status mkv_attn_prefill(mkv_cache *h, int layer, uint32_t first_pos, uint32_
         set_error("f16 queries go with the f16 cache (q_f16 + attn_fa_mx); the f32 cache's attn_fa / attn_fd4 read f32 queries");
         return MKV_ERR_UNSUPPORTED;
     }
-    // f32 cache, two ways. prefill_f32_tc.cu takes 32 tokens at a time: about 27 us a layer and 1.3 us per 1,000 keys and 32
-    // tokens. Batched verify items take 4 tokens: about 12 us and 0.65 us per 1,000 keys and 4 tokens, so they win for a few
-    // tokens. Measured, us a layer, items / kernel: 5 tokens over 4,096 16 / 32, 16 over 4,096 22 / 34, 16 over 8,192 33 / 38,
-    // 32 over 4,096 36 / 34, 16 over 32,768 95 / 70, 64 over 1,000 30 / 33, 64 over 4,096 70 / 36, 512 over 4,096 567 / 124.
+    // f32 cache, two ways. prefill_f32_tc.cu takes 32 tokens at a time: about 19 us a layer and 1.25 us per 1,000 keys and 32
+    // tokens. Batched verify items take 4 tokens: about 15 us, from some thousand keys on 0.65 us per 1,000 keys and 4 tokens; more
+    // than 16 of them are staged with a copy in the stream. Measured, us a layer, items / kernel: 8 tokens over 32,000 49 / 59,
+    // 12 over 8,192 27 / 30, over 16,000 43 / 41; 16 over 4,096 20 / 23, over 8,192 32 / 31; 32 over 2,000 20 / 20, over 4,096
+    // 31 / 25; 40 over 1,000 20 / 21, over 2,000 26 / 21; 64 over 500 20 / 20; 96 over 16 28 / 17; 300 over 4,096 466 / 89.
     const uint32_t g4 = (ntok + 3u) / 4u, g32 = (ntok + 31u) / 32u;
-    if (g4 > 2u * g32 && (uint64_t)(g4 - 2u * g32) * (end - first_pos) >= 23000u)
+    if (g4 > PARAM_ITEMS || (g4 > 2u * g32 && (uint64_t)(g4 - 2u * g32) * (end - first_pos) >= 12000u))
         return launch_prefill_f32_tc(c->ctx, c, layer, first_pos, pos0, ntok, q, out);
     // groups of up to 4 tokens through the f32 verify kernel (the reference's attn_fd4 also reads
     // K/V once per 4 tokens, W/ops.wgsl:694-699), one ragged batch per <= SLOT_ITEMS groups

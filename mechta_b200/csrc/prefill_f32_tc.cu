@@ -11,10 +11,11 @@
 // accumulated first, so that the truncations of the long chain happen on small sums.
 //
 // The f32 prefill used to run as batched 4-token verify items, which read every key once per 4 tokens: 512 tokens over a
-// 4,096-token prefix took 567 us a layer, here 124 (8,000: 951 -> 203, 32,768: 3,380 -> 740). A tile needs 6,144 tensor core
-// cycles (three products of 128 x 128 x 256 twice), about 5,000 issue slots of conversion, softmax and folding, and 128 KB of
-// L2 -> SM traffic a CTA. What is not overlapped is the softmax between a tile's two products: tensor memory has no room for
-// a second S beside O_t, Q and P. Relative error against f64 over 5 ... 512 tokens and 16 ... 32,768 keys: 3.6e-7 to 6.7e-7
+// 4,096-token prefix took 567 us a layer, here 123 (8,000: 951 -> 200, 32,768: 3,380 -> 710). A tile takes about 10,400 cycles, of
+// which 9,500 are the products: 48 of 256 x 128 x 16 at 128 cycles each (by a pair of CTAs, N = 128 runs at half the rate of N =
+// 256) and 24 of 256 x 256 x 16 at 140. The rest is the softmax between a tile's two products: tensor memory has no room for a
+// second S, or for one of 256 keys, beside O_t, Q and P. Starting P.V on the first half of the weights was 2 % faster and took
+// the error from 6.5e-7 to 7.8e-7. Relative error against f64 over 5 ... 512 tokens and 16 ... 32,768 keys: 3.6e-7 to 6.7e-7
 // (2-norm), the verify items 6.5e-7 to 1.1e-6.
 //
 // Memory. TMA brings a slot [64 keys][128 dims] f32 (32 KB) as two regions of 64 dims, each two boxes of [64 keys][32 dims]

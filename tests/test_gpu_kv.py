@@ -746,8 +746,9 @@ def test_prefill_f16_tile_and_split_edges(ctx, oracle, prefix, ntok, first, q16)
     cache.close()
 
 
-@pytest.mark.parametrize("prefix,ntok,first", [(23000, 12, 0), (22983, 12, 0), (11497, 13, 0), (12000, 33, 10000), (3802, 32, 0), (1810, 64, 0),
-                                                (1791, 97, 70), (700, 129, 0), (383, 257, 129), (63, 448, 0), (40, 2400, 0), (8000, 300, 7500)])
+@pytest.mark.parametrize("prefix,ntok,first", [(11988, 12, 0), (11987, 12, 0), (5987, 13, 0), (12000, 33, 10000), (1968, 32, 0), (1967, 32, 0),
+                                                (936, 64, 0), (0, 65, 0), (1791, 97, 70), (383, 257, 129), (63, 448, 0), (40, 2400, 0),
+                                                (8000, 300, 7500)])
 def test_prefill_f32_tile_and_split_edges(ctx, oracle, prefix, ntok, first):
     """The f32 prefill at the line between batched verify items and the kernel of its own (number of 4-token groups times keys), and
     that kernel at the edges of its key tiles (128, converted in halves of 64), token groups (32 a pair of CTAs) and of the split
@@ -755,7 +756,8 @@ def test_prefill_f32_tile_and_split_edges(ctx, oracle, prefix, ntok, first):
     fmt = kv.KvFormat.F32
     cache = kv.KvCache(ctx, fmt, 1, (prefix + ntok + 4096) // 1024 * 1024)
     kc, vc = fill_both(oracle, cache, 0, prefix + ntok, 400 + ntok)
-    own = ((ntok + 3) // 4 - 2 * ((ntok + 31) // 32)) * (prefix + ntok - first) >= 23000  # goes to the kernel of its own
+    # goes to the kernel of its own
+    own = ntok > 64 or ((ntok + 3) // 4 - 2 * ((ntok + 31) // 32)) * (prefix + ntok - first) >= 12000
     for t in cache.buffer_tensors(0) if own else ():
         t[prefix + ntok:] = float("nan")
     q = synth.normal(401, synth.S_Q, ntok, (ntok, 16, 256))
