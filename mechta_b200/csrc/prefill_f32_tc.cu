@@ -1,6 +1,6 @@
 // Prefill attention over the f32 cache, f32-grade arithmetic on the tensor cores: tcgen05.mma by CTA pairs.
 //
-// Stands in for attn_fa / attn_fd4 + attn_fd_combine of the reference on the f32 cache (W/ops.wgsl:600-760): token T of the
+// Stands in for attn_fa / attn_fd4 + attn_fd_combine of the reference on the f32 cache (W/ops.wgsl:562-651,711-778): token T of the
 // block (at pos0 + T) sees first_pos <= key < pos0 + 1 + T. The work is cut as in prefill_tc.cu (prefill_plan.cuh): an item is
 // 32 tokens x the 8 query heads of one KV head = 256 rows, 128 in each CTA of a pair, tiles of 128 keys, each CTA loading one
 // half of a tile (64 keys of K, 128 of the 256 dims of V); parts of split items are merged by the same kernel.
@@ -519,8 +519,6 @@ mkv_status prefill_f32_tc_setup_device() {
 
 mkv_status launch_prefill_f32_tc(Ctx *ctx, Cache *c, int layer, uint32_t first_pos, uint32_t pos0, uint32_t ntok, const float *q, float *out) {
     const PfPlan plan = pf_plan(ctx, PS_COST, first_pos, pos0, ntok);
-    mkv_status st = prefill_scratch(ctx);
-    if (st != MKV_OK) return st;
     const CUtensorMap &km = c->maps_host[2 * (c->n_layers + layer)], &vm = c->maps_host[2 * (c->n_layers + layer) + 1];
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2u * plan.pairs);

@@ -77,10 +77,10 @@ __host__ __device__ inline size_t pf_slot(uint32_t pair, uint32_t piece, uint32_
 struct PfCost {
     float segment, merge, part;
 };
+// The plan of a launch, with the context's scratch of two partials per CTA in place if the plan needs it. The scratch is allocated
+// for the context's first launch that splits items and kept until the context goes; where it cannot be had (no memory left, or the
+// stream is being captured) items stay whole.
 PfPlan pf_plan(Ctx *ctx, const PfCost &cost, uint32_t first_pos, uint32_t pos0, uint32_t ntok);
-// Scratch of the split items: two partials per CTA, allocated with the context's first prefill launch and kept until the
-// context goes.
-mkv_status prefill_scratch(Ctx *ctx);
 // Merges the split items of the launch in front, if it has any.
 mkv_status launch_prefill_merge(Ctx *ctx, const PfPlan &plan, float *out);
 

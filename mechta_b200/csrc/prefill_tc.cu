@@ -539,15 +539,25 @@ mkv_status prefill_tc_setup_device() {
     return MKV_OK;
 }
 
-mkv_status prefill_scratch(Ctx *ctx) {
-    if (ctx->pf_scratch) return MKV_OK;
-    const size_t bytes = 2u * (size_t)ctx->sm_count * PF_PART * sizeof(float);
-    if (cudaMalloc(&ctx->pf_scratch, bytes) != cudaSuccess) {
-        cudaGetLastError();
-        set_error("out of device memory for the prefill partials (%zu bytes)", bytes);
-        return MKV_ERR_NOMEM;
+static bool pf_splits(const PfPlan &plan) {
+    if (plan.per > 1u) return plan.part_len(plan.tiles_of(0)) < plan.tiles_of(0);
+    for (uint32_t i = 0, base = 0; plan.per == 0u && i < plan.nitems; i++) {
+        const uint32_t n = plan.tiles_of(i);
+        if (base / plan.len != (base + n - 1u) / plan.len) return true;
+        base += n;
     }
-    return MKV_OK;
+    return false;
+}
+
+static bool pf_scratch(Ctx *ctx) {
+    if (ctx->pf_scratch) return true;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone &&
+        cudaMalloc(&ctx->pf_scratch, 2u * (size_t)ctx->sm_count * PF_PART * sizeof(float)) == cudaSuccess)
+        return true;
+    cudaGetLastError();
+    ctx->pf_scratch = nullptr;
+    return false;
 }
 
 // Chooses the way of the three that the cost model expects to be the fastest. Whole items need no merge but leave pairs idle
@@ -595,18 +605,15 @@ PfPlan pf_plan(Ctx *ctx, const PfCost &cost, uint32_t first_pos, uint32_t pos0, 
             plan.pairs = per * n;
         }
     }
+    if (pf_splits(plan) && !pf_scratch(ctx)) {
+        plan.per = 1;
+        plan.pairs = std::min(n, npairs);
+    }
     return plan;
 }
 
 mkv_status launch_prefill_merge(Ctx *ctx, const PfPlan &plan, float *out) {
-    bool split = false;
-    for (uint32_t i = 0, base = 0; plan.per == 0u && i < plan.nitems && !split; i++) {
-        const uint32_t n = plan.tiles_of(i);
-        split = base / plan.len != (base + n - 1u) / plan.len;
-        base += n;
-    }
-    if (plan.per > 1u) split = plan.part_len(plan.tiles_of(0)) < plan.tiles_of(0);
-    if (!split) return MKV_OK;
+    if (!pf_splits(plan)) return MKV_OK;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(64u, plan.nitems);
     cfg.blockDim = dim3(256);
@@ -629,8 +636,6 @@ mkv_status launch_prefill_f16_tc(Ctx *ctx, Cache *c, int layer, uint32_t first_p
     const uint32_t phase = 0u;
 #endif
     const PfPlan plan = pf_plan(ctx, TC_COST, first_pos, pos0, ntok);
-    mkv_status st = prefill_scratch(ctx);
-    if (st != MKV_OK) return st;
     const CUtensorMap &km = c->maps_host[2 * (c->n_layers + layer)], &vm = c->maps_host[2 * (c->n_layers + layer) + 1];
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2u * plan.pairs);

@@ -772,6 +772,32 @@ def test_prefill_f32_tile_and_split_edges(ctx, oracle, prefix, ntok, first):
     cache.close()
 
 
+@pytest.mark.parametrize("fmt", FMTS)
+def test_first_prefill_of_a_context_under_capture(fmt):
+    """A launch that would split its items, captured before the context has the scratch for it, keeps them whole; the graph's result
+    is that of the split launch but for the order of sums."""
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        own = kv.KvContext(0, stream)
+        cache = kv.KvCache(own, fmt, 1, 6144)
+        for t in cache.buffer_tensors(0):
+            t[:5040].normal_()
+        cache.set_len(5040)
+        q = torch.randn(40, 16, 256, device="cuda")
+        out, want = torch.empty_like(q), torch.empty_like(q)
+        own.sync()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            cache.attn_prefill(0, 0, 5000, q, out)
+        graph.replay()
+        cache.attn_prefill(0, 0, 5000, q, want)
+        own.sync()
+    assert ((out - want).norm() / want.norm()).item() < (1e-3 if fmt == kv.KvFormat.F16 else 2e-6)
+    del graph
+    cache.close()
+    own.close()
+
+
 # ---------------------------------------------------------------- snapshot / restore ---------------------------
 
 @pytest.mark.parametrize("fmt", FMTS)
