@@ -11,7 +11,7 @@
 // accumulated first, so that the truncations of the long chain happen on small sums.
 //
 // The f32 prefill used to run as batched 4-token verify items, which read every key once per 4 tokens: 512 tokens over a
-// 4,096-token prefix took 567 us a layer, here 123 (8,000: 951 -> 200, 32,768: 3,380 -> 710). A tile takes about 10,400 cycles, of
+// 4,096-token prefix took 567 us a layer, here 120 (8,000: 951 -> 200, 32,768: 3,380 -> 710). A tile takes about 10,400 cycles, of
 // which 9,500 are the products: 48 of 256 x 128 x 16 at 128 cycles each (by a pair of CTAs, N = 128 runs at half the rate of N =
 // 256) and 24 of 256 x 256 x 16 at 140. The rest is the softmax between a tile's two products: tensor memory has no room for a
 // second S, or for one of 256 keys, beside O_t, Q and P. Starting P.V on the first half of the weights was 2 % faster and took
