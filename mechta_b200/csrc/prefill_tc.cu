@@ -133,7 +133,10 @@ prefill_f16_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
                 const uint32_t end = plan.pos0 + plan.item_end(sg.item); // no key at or past this one is seen by the item's tokens
                 for (uint32_t j = sg.a; j < sg.b; j++, g++) {
                     const uint32_t s = g % TC_NST, key0 = (plan.t0 + j) * PF_KEYS;
-                    const int y[2] = {(int)(key0 - row0), key0 + 64u < end ? (int)(key0 + 64u - row0) : TC_ROW_OUTSIDE};
+                    // A half tile without a key for any of the item's tokens is not read: its weights are zero, but zero times
+                    // an infinity or NaN left in such a V row is not. (The first half can only lie below first_pos.)
+                    const int y[2] = {key0 + 64u > plan.first_pos ? (int)(key0 - row0) : TC_ROW_OUTSIDE,
+                                      key0 + 64u < end ? (int)(key0 + 64u - row0) : TC_ROW_OUTSIDE};
                     const uint32_t par = ((g / TC_NST) - 1u) & 1u;
                     if (g >= (uint32_t)TC_NST && !(ok = tc_wait(bar_k_empty + 8u * s, par, sh, status))) break;
                     // both CTAs' halves are counted on the first CTA's barrier: its MMA thread is the one that waits

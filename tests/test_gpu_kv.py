@@ -746,6 +746,39 @@ def test_prefill_f16_tile_and_split_edges(ctx, oracle, prefix, ntok, first, q16)
     cache.close()
 
 
+def prefill_clean_and_poisoned(ctx, fmt, prefix, ntok, first, rows, seed):
+    """Outputs of a block over N(0,1) rows, before and after the V rows in `rows` became infinite or NaN."""
+    cache = kv.KvCache(ctx, fmt, 1, (prefix + ntok + 4096) // 1024 * 1024)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    k, v = cache.buffer_tensors(0)
+    for t in (k, v):
+        t[:prefix + ntok].normal_(generator=g)
+    cache.set_len(prefix + ntok)
+    q = torch.randn(ntok, 16, 256, device="cuda", generator=g)
+    out = [torch.empty_like(q) for _ in range(2)]
+    cache.attn_prefill(0, first, prefix, q, out[0])
+    ctx.sync()
+    v[rows[0]:rows[1]] = float("inf")
+    v[rows[0]:rows[1]:2] = float("nan")
+    cache.attn_prefill(0, first, prefix, q, out[1])
+    ctx.sync()
+    cache.close()
+    assert torch.isfinite(out[0]).all()
+    return out
+
+
+@pytest.mark.parametrize("fmt", FMTS)
+@pytest.mark.parametrize("prefix,ntok,first", [(2000, 40, 1000), (200, 70, 64), (9000, 200, 127), (9000, 100, 8959), (300, 3, 255)])
+def test_prefill_does_not_read_half_tiles_below_first_pos(ctx, fmt, prefix, ntok, first):
+    """first_pos in the second half of a 128-key tile: what the V rows of the first half hold, NaN and infinities too, does not reach
+    the outputs (their weights are zero, but zero times NaN is not)."""
+    lo = first // 128 * 128
+    assert first - lo >= 64
+    clean, poisoned = prefill_clean_and_poisoned(ctx, fmt, prefix, ntok, first, (lo, lo + 64), 500 + first)
+    assert torch.equal(clean, poisoned)
+
+
 @pytest.mark.parametrize("prefix,ntok,first", [(11988, 12, 0), (11987, 12, 0), (5987, 13, 0), (12000, 33, 10000), (1968, 32, 0), (1967, 32, 0),
                                                 (936, 64, 0), (0, 65, 0), (1791, 97, 70), (383, 257, 129), (63, 448, 0), (40, 2400, 0),
                                                 (8000, 300, 7500)])
