@@ -196,24 +196,24 @@ prefill_f32_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
                 tc_commit2(bar_s_full);
                 return true;
             };
-            auto pv = [&]() -> bool { // O_t = P V for tile g, from zero
+            // O_t = P V for tile g, from zero. mma(a, b, accumulate, key) issues one MMA over the 16 keys from `key`; key0 = the tile's first.
+            auto pv = [&](uint32_t key0, auto mma) -> bool {
 #pragma unroll 1
                 for (uint32_t s = 0; s < 2u; s++) {
                     if (!slot_wait(4u * g + 2u + s)) return false;
-                    const uint32_t v = slot(4u * g + 2u + s), p = S + 64u * s;
+                    const uint32_t v = slot(4u * g + 2u + s), p = S + 64u * s, key = key0 + 64u * s;
 #pragma unroll
-                    for (uint32_t ks = 0; ks < 4u; ks++) { // 16 keys per MMA: weights' hi halves in 8 columns, lo halves in the next 8
+                    for (uint32_t ks = 0; ks < 4u; ks++) { // weights' hi halves in 8 columns, lo halves in the next 8
                         // V slot, N-major: the next 64 dims one region on, the next 8 keys 1024 bytes on
-                        tc_mma2_f16_ta(O, p + 16u * ks + 8u, tc_desc_sw128(v + ks * 2048u, PS_REGION, 1024), IDESC_PV, s | ks);
-                        tc_mma2_f16_ta(O, p + 16u * ks, tc_desc_sw128(v + PS_BLK + ks * 2048u, PS_REGION, 1024), IDESC_PV, 1u);
+                        mma(p + 16u * ks + 8u, tc_desc_sw128(v + ks * 2048u, PS_REGION, 1024), s | ks, key + 16u * ks);
+                        mma(p + 16u * ks, tc_desc_sw128(v + PS_BLK + ks * 2048u, PS_REGION, 1024), 1u, key + 16u * ks);
                     }
                 }
 #pragma unroll 1
                 for (uint32_t s = 0; s < 2u; s++) {
-                    const uint32_t v = slot(4u * g + 2u + s), p = S + 64u * s;
+                    const uint32_t v = slot(4u * g + 2u + s), p = S + 64u * s, key = key0 + 64u * s;
 #pragma unroll
-                    for (uint32_t ks = 0; ks < 4u; ks++)
-                        tc_mma2_f16_ta(O, p + 16u * ks, tc_desc_sw128(v + ks * 2048u, PS_REGION, 1024), IDESC_PV, 1u);
+                    for (uint32_t ks = 0; ks < 4u; ks++) mma(p + 16u * ks, tc_desc_sw128(v + ks * 2048u, PS_REGION, 1024), 1u, key + 16u * ks);
                     tc_commit2(bar_empty + 8u * ((4u * g + 2u + s) % PS_NSLOT));
                 }
                 tc_commit2(bar_o_full);
@@ -226,6 +226,7 @@ prefill_f32_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
                 if (!(ok = ps_wait(bar_q_full, nseg & 1u, sh, status))) break; // the segment's queries are in place
                 tc_fence_after();
                 nseg++;
+                const uint32_t tok_pos = plan.pos0 + 32u * plan.group_of(sg.item);
                 for (uint32_t j = sg.a; j < sg.b; j++, g++) {
                     // The products run in the order in which they are issued: S of this tile overwrites weights that the product
                     // before has read. The weights of this tile are there once its scores have been read and O_t of the tile
@@ -233,7 +234,14 @@ prefill_f32_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
                     if (!(ok = qk())) break;
                     if (!(ok = ps_wait(bar_p_full, g & 1u, sh, status))) break;
                     tc_fence_after();
-                    if (!(ok = pv())) break;
+                    const uint32_t key0 = (plan.t0 + j) * PF_KEYS;
+                    if (key0 + PF_KEYS <= tok_pos + 1u) // every token sees the whole tile
+                        ok = pv(key0, [&](uint32_t a, uint64_t b, uint32_t acc, uint32_t) { tc_mma2_f16_ta(O, a, b, IDESC_PV, acc); });
+                    else
+                        ok = pv(key0, [&](uint32_t a, uint64_t b, uint32_t acc, uint32_t key) {
+                            tc_mma2_f16_ta_off(O, a, b, IDESC_PV, acc, pf_blind_rows(key, tok_pos), pf_blind_rows(key, tok_pos + 16u));
+                        });
+                    if (!ok) break;
                 }
             }
         }
@@ -366,7 +374,7 @@ prefill_f32_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
                 ok = __all_sync(0xffffffffu, ps_wait(bar_s_full, g & 1u, sh, status)) && ok;
                 tc_fence_after();
                 const uint32_t s_addr = tmem + lane_addr + PS_COL_S + 64u * half;
-                const uint32_t key_base = (plan.t0 + j) * PF_KEYS + 64u * half;
+                const uint32_t tile_key = (plan.t0 + j) * PF_KEYS, key_base = tile_key + 64u * half;
                 // which of the 64 keys the row sees: all of them off the causal diagonal and the window start
                 const bool masked = key_base + 64u > full_below || key_base < plan.first_pos;
                 const uint32_t k_lo = plan.first_pos > key_base ? plan.first_pos - key_base : 0u;
@@ -448,8 +456,10 @@ prefill_f32_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
                         uint32_t o[32];
                         tmem_ld32(tmem + lane_addr + PS_COL_O + 128u * half + 32u * c, o);
                         tmem_wait_ld();
+                        if (vis > tile_key) { // (no product has written the row of a token that sees none of the tile)
 #pragma unroll
-                        for (uint32_t i = 0; i < 32u; i++) acc[32u * c + i] += __uint_as_float(o[i]);
+                            for (uint32_t i = 0; i < 32u; i++) acc[32u * c + i] += __uint_as_float(o[i]);
+                        }
                     }
                 }
                 tc_fence_before();

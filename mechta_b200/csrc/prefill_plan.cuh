@@ -66,6 +66,14 @@ struct PfWalk {
         return false;
     }
 };
+// The rows of a CTA whose tokens see none of the keys from `key` on, as lanes of a group of 32 (rows are head * 16 + token, so a group
+// is two heads of the same 16 tokens); tok_pos = position of the CTA's first token. P V leaves these rows out, 16 keys at a time
+// (the K of one MMA): their weights are zero, but zero times an infinity or NaN in a later token's V row, or in a row past the
+// block, is not.
+__device__ __forceinline__ uint32_t pf_blind_rows(uint32_t key, uint32_t tok_pos) {
+    const uint32_t m = (1u << (key > tok_pos ? min(key - tok_pos, 16u) : 0u)) - 1u;
+    return m | m << 16;
+}
 // Where a pair's CTA keeps the partial of a part: a pair has at most one segment that continues an item begun by the pair
 // before it (slot 0) and at most one that begins an item it does not finish (slot 1).
 __host__ __device__ inline size_t pf_slot(uint32_t pair, uint32_t piece, uint32_t cta) {

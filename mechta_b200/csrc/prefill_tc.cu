@@ -27,7 +27,8 @@
 // memory); the row's threads read S, release it (so that the next tile's S is computed while this one is in softmax), scale,
 // mask, exponentiate against a reference maximum that only moves when the tile exceeds it by more than 8 (the reference's
 // lazy maximum, M/dmx.rs:80 and W/fa_mx.wgsl:120: a matrix accumulator cannot be rescaled per row cheaply), write P as f16 to
-// shared memory; O += P V (8 MMAs, V used N-major straight from its TMA tile).
+// shared memory; O += P V (8 MMAs, V used N-major straight from its TMA tile). Rows that see none of an MMA's 16 keys are left out of
+// it (pf_blind_rows); a row that sees no key of a segment has l = 0 there and its O, which no product has written, is not used.
 // TMEM: O = columns 0..255, S = 256..383, Q (f16) = 384..511. Every wait is bounded; TMEM is freed on every path.
 #include <stdlib.h>
 
@@ -190,9 +191,14 @@ prefill_f16_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
                 if (!(ok = tc_wait(bar_q_full, nseg & 1u, sh, status))) break;
                 tc_fence_after();
                 nseg++;
-                const uint32_t n = sg.b - sg.a;
+                const uint32_t n = sg.b - sg.a, tok_pos = plan.pos0 + 32u * plan.group_of(sg.item);
                 if (!(ok = qk(g))) break;
-                for (uint32_t j = 0; j < n; j++, g++) {
+                // Tiles of which every token sees all keys, then the one or two at the item's end, where an MMA leaves out the rows
+                // that see none of its 16 keys and MMAs that no row has a share in are not issued. (With one loop for both, ten layers
+                // of 2,048 tokens over 32,768 took 1.5 % longer; leaving rows out in every MMA, 7 %.)
+                const uint32_t whole = min(n, max((tok_pos + 1u) / PF_KEYS, plan.t0 + sg.a) - (plan.t0 + sg.a));
+                uint32_t j = 0;
+                for (; j < whole; j++, g++) {
                     if (j + 1u < n && !(ok = qk(g + 1u))) break; // the next tile's scores while this one is in softmax
                     const uint32_t s = g % TC_NST;
                     if (!(ok = tc_wait(bar_v_full + 8u * s, (g / TC_NST) & 1u, sh, status))) break;
@@ -208,6 +214,28 @@ prefill_f16_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
                     }
                     tc_commit2(bar_v_empty + 8u * s);
                     tc_commit2(bar_pv_done); // O holds the segment's tiles so far; P may be overwritten
+                }
+                for (; ok && j < n; j++, g++) {
+                    if (j + 1u < n && !(ok = qk(g + 1u))) break;
+                    const uint32_t s = g % TC_NST;
+                    if (!(ok = tc_wait(bar_v_full + 8u * s, (g / TC_NST) & 1u, sh, status))) break;
+                    if (!(ok = tc_wait(bar_p_full, g & 1u, sh, status))) break;
+                    tc_fence_after();
+                    const uint32_t vb = smem_base + TC_OFF_V + s * TC_HALF, pb = smem_base + TC_OFF_P;
+#pragma unroll 1
+                    for (uint32_t ks = 0; ks < 8u; ks++) {
+                        const uint32_t key = (plan.t0 + sg.a + j) * PF_KEYS + 16u * ks;
+                        if (key > tok_pos + 31u) break;
+                        const uint32_t off0 = pf_blind_rows(key, tok_pos), off1 = pf_blind_rows(key, tok_pos + 16u);
+                        const uint64_t a = tc_desc_sw128(pb + (ks >> 2) * 16384u + (ks & 3u) * 32u, 16, 1024);
+                        const uint64_t b = tc_desc_sw128(vb + ks * 2048u, 2u * TC_BOX, 1024);
+                        const uint32_t acc = (j > 0 || ks > 0) ? 1u : 0u;
+                        if (phase == 1u) continue;
+                        if ((off0 | off1) == 0u) tc_mma2_f16(tmem + TC_COL_O, a, b, IDESC_PV, acc);
+                        else tc_mma2_f16_off(tmem + TC_COL_O, a, b, IDESC_PV, acc, off0, off1);
+                    }
+                    tc_commit2(bar_v_empty + 8u * s);
+                    tc_commit2(bar_pv_done);
                 }
             }
         }
@@ -496,6 +524,12 @@ prefill_merge_kernel(const __grid_constant__ PfPlan plan, const float *__restric
                 v[k][i] = s < np && real ? __ldcg(reinterpret_cast<const float4 *>(ps + ((size_t)(8u * eighth + 4u * ch + i) * 128u + row) * 4u))
                                  : make_float4(0.f, 0.f, 0.f, 0.f);
         }
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (ml[k].y == 0.0f) { // the row's token sees no key of the part: no product has written its O
+#pragma unroll
+                for (int i = 0; i < 4; i++) v[k][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
         const float mx = fmaxf(fmaxf(ml[0].x, ml[1].x), fmaxf(ml[2].x, ml[3].x));
         if (mx > M) {
             const float f = M > NEG_TEST ? exp2f(M - mx) : 0.0f;
@@ -572,6 +606,9 @@ prefill_merge_few_kernel(const __grid_constant__ PfPlan plan, const float *__res
             v[k] = s < np && real ? __ldcg(reinterpret_cast<const float4 *>(ps + ((size_t)(8u * eighth + ch) * 128u + row) * 4u))
                                   : make_float4(0.f, 0.f, 0.f, 0.f);
         }
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (ml[k].y == 0.0f) v[k] = make_float4(0.f, 0.f, 0.f, 0.f); // the row's token sees no key of the part: no product has written its O
         const float mx = fmaxf(fmaxf(ml[0].x, ml[1].x), fmaxf(ml[2].x, ml[3].x));
         if (mx > M) {
             const float f = M > NEG_TEST ? exp2f(M - mx) : 0.0f;

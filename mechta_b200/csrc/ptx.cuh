@@ -219,6 +219,26 @@ __device__ __forceinline__ void tc_mma2_f16_ta(uint32_t d_tmem, uint32_t a_tmem,
         "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// The same with some rows of D left as they are: off0 / off1 name lanes to skip in the first / second CTA, one bit a lane, and hold
+// for each group of 32 lanes alike.
+__device__ __forceinline__ void tc_mma2_f16_off(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate,
+                                                uint32_t off0, uint32_t off1) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %6, %6, %6, %6}, p;\n\t}" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(off0), "r"(off1)
+        : "memory");
+}
+__device__ __forceinline__ void tc_mma2_f16_ta_off(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate,
+                                                   uint32_t off0, uint32_t off1) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5, %6, %6, %6, %6}, p;\n\t}" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(off0), "r"(off1)
+        : "memory");
+}
 // The barrier at this offset in both CTAs gets one arrival once every MMA issued so far by this thread has completed.
 __device__ __forceinline__ void tc_commit2(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),

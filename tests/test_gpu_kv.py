@@ -779,6 +779,19 @@ def test_prefill_does_not_read_half_tiles_below_first_pos(ctx, fmt, prefix, ntok
     assert torch.equal(clean, poisoned)
 
 
+@pytest.mark.parametrize("fmt", FMTS)
+@pytest.mark.parametrize("prefix,ntok,row", [(2024, 32, 2056), (2024, 96, 2050), (2032, 200, 2048), (2017, 100, 2048), (5000, 300, 5121),
+                                             (5000, 300, 5299), (9001, 200, 9201), (33, 400, 300), (0, 65, 64), (30011, 65, 30076)])
+def test_prefill_tokens_do_not_feel_later_rows(ctx, fmt, prefix, ntok, row):
+    """A NaN or infinite V row, a later token's or one past the block, reaches only tokens whose position lies in the row's own group of
+    16 keys or behind it (16 keys are one MMA, in which a weight of zero meets the row); all others keep their bits."""
+    clean, poisoned = prefill_clean_and_poisoned(ctx, fmt, prefix, ntok, 0, (row, row + 1), 600 + row)
+    safe = min(ntok, max(0, row // 16 * 16 - prefix))
+    assert safe > 0 and torch.equal(clean[:safe], poisoned[:safe])
+    seen = row - prefix  # the token that the row belongs to sees it
+    assert seen >= ntok or not torch.isfinite(poisoned[seen:]).any(dim=-1).any()
+
+
 @pytest.mark.parametrize("prefix,ntok,first", [(11988, 12, 0), (11987, 12, 0), (5987, 13, 0), (12000, 33, 10000), (1968, 32, 0), (1967, 32, 0),
                                                 (936, 64, 0), (0, 65, 0), (1791, 97, 70), (383, 257, 129), (63, 448, 0), (40, 2400, 0),
                                                 (8000, 300, 7500)])
