@@ -70,7 +70,8 @@ mkv_status mkv_sync(mkv_ctx *ctx);
 uint64_t mkv_launch_count(const mkv_ctx *ctx);
 /* Kernel timing with CUDA events on the compute stream, off by default. While on, every attention core
  * kernel (verify / prefill) is bracketed by two events; mkv_prof_read blocks on the last one and returns
- * the summed milliseconds and the number of launches since the last read, then clears them. Mirrors the
+ * the summed milliseconds and the number of launches since the last read, then clears them. A prefill kernel and
+ * the small kernel that merges its split items count as one launch. Mirrors the
  * reference's per-dispatch GPU timestamps of "attn.core" (M/engine.rs:1274-1295). on = 0 switches it off;
  * on > 0 switches it on and creates that many event pairs ahead of time (more are created as needed). */
 mkv_status mkv_prof_enable(mkv_ctx *ctx, int on);

@@ -119,6 +119,22 @@ static mkv_status check_device_status(Ctx *ctx) {
     return MKV_OK;
 }
 
+mkv_status prof_begin(Ctx *ctx) {
+    if (!ctx->prof) return MKV_OK;
+    if (ctx->prof_used == ctx->prof_events.size()) {
+        cudaEvent_t a, b;
+        MKV_CUDA(cudaEventCreate(&a));
+        MKV_CUDA(cudaEventCreate(&b));
+        ctx->prof_events.push_back({a, b});
+    }
+    MKV_CUDA(cudaEventRecord(ctx->prof_events[ctx->prof_used].first, ctx->stream));
+    return MKV_OK;
+}
+mkv_status prof_end(Ctx *ctx) {
+    if (ctx->prof) MKV_CUDA(cudaEventRecord(ctx->prof_events[ctx->prof_used++].second, ctx->stream));
+    return MKV_OK;
+}
+
 // ---- guarded allocations (the checked build, -DMKV_CHECKS) ---------------------------------------------------
 // Every buffer of a cache (the K and V rows of each layer, the split-K pieces) is bracketed by GUARD bytes of a canary
 // pattern that no kernel may touch; mkv_cache_check_guards counts the bytes that changed. The shipped build allocates
@@ -1093,8 +1109,10 @@ mkv_status mkv_attn_prefill(mkv_cache *h, int layer, uint32_t first_pos, uint32_
             set_error("the warp-MMA baseline kernel (MKV_PREFILL=mma) takes f32 queries only");
             return MKV_ERR_UNSUPPORTED;
         }
-        return use_mma ? launch_prefill_f16_mma(c->ctx, c, layer, first_pos, pos0, ntok, q, out)
-                       : launch_prefill_f16_tc(c->ctx, c, layer, first_pos, pos0, ntok, qv, q_is_f16 != 0, out);
+        if ((st = prof_begin(c->ctx)) != MKV_OK) return st;
+        st = use_mma ? launch_prefill_f16_mma(c->ctx, c, layer, first_pos, pos0, ntok, q, out)
+                     : launch_prefill_f16_tc(c->ctx, c, layer, first_pos, pos0, ntok, qv, q_is_f16 != 0, out);
+        return st == MKV_OK ? prof_end(c->ctx) : st;
     }
     if (q_is_f16) {
         set_error("f16 queries go with the f16 cache (q_f16 + attn_fa_mx); the f32 cache's attn_fa / attn_fd4 read f32 queries");
@@ -1106,8 +1124,11 @@ mkv_status mkv_attn_prefill(mkv_cache *h, int layer, uint32_t first_pos, uint32_
     // 12 over 8,192 27 / 30, over 16,000 43 / 41; 16 over 4,096 20 / 23, over 8,192 32 / 31; 32 over 2,000 20 / 20, over 4,096
     // 31 / 25; 40 over 1,000 20 / 21, over 2,000 26 / 21; 64 over 500 20 / 20; 96 over 16 28 / 17; 300 over 4,096 466 / 89.
     const uint32_t g4 = (ntok + 3u) / 4u, g32 = (ntok + 31u) / 32u;
-    if (g4 > PARAM_ITEMS || (g4 > 2u * g32 && (uint64_t)(g4 - 2u * g32) * (end - first_pos) >= 12000u))
-        return launch_prefill_f32_tc(c->ctx, c, layer, first_pos, pos0, ntok, q, out);
+    if (g4 > PARAM_ITEMS || (g4 > 2u * g32 && (uint64_t)(g4 - 2u * g32) * (end - first_pos) >= 12000u)) {
+        if ((st = prof_begin(c->ctx)) != MKV_OK) return st;
+        st = launch_prefill_f32_tc(c->ctx, c, layer, first_pos, pos0, ntok, q, out);
+        return st == MKV_OK ? prof_end(c->ctx) : st;
+    }
     // groups of up to 4 tokens through the f32 verify kernel (the reference's attn_fd4 also reads
     // K/V once per 4 tokens, W/ops.wgsl:694-699), one ragged batch per <= SLOT_ITEMS groups
     uint32_t done = 0;

@@ -214,6 +214,10 @@ mkv_status launch_step_prep(Ctx *ctx, mkv_fmt fmt, const float *qf, const float 
                             uint32_t row_first, uint32_t capacity, uint32_t ring, uint32_t pos, uint32_t ntok);
 // a shard without any visible key: its (empty) record rows still go to every rank, and the ranks' rows are merged into `out`
 mkv_status launch_exchange_empty(Ctx *ctx, const PushInfo *push, uint32_t epoch, uint32_t ntok, float *out);
+// The next pair of timing events (mkv_prof_enable): prof_begin records the first in front of an attention core launch, prof_end the
+// second behind it. Both do nothing while timing is off.
+mkv_status prof_begin(Ctx *ctx);
+mkv_status prof_end(Ctx *ctx);
 // plans the split of the items so that the grid fills the SMs once
 void plan_items(Ctx *ctx, mkv_fmt fmt, VerifyItem *items, int n);
 

@@ -549,19 +549,8 @@ mkv_status launch_verify(Ctx *ctx, mkv_fmt fmt, VerifyItem *items_host, int n, b
         memset(&single.kmap, 0, sizeof single.kmap);
         memset(&single.vmap, 0, sizeof single.vmap);
     }
-    cudaEvent_t e1 = nullptr;
-    if (ctx->prof) {
-        if (ctx->prof_used == ctx->prof_events.size()) {
-            cudaEvent_t a, b;
-            MKV_CUDA(cudaEventCreate(&a));
-            MKV_CUDA(cudaEventCreate(&b));
-            ctx->prof_events.push_back({a, b});
-        }
-        const cudaEvent_t e0 = ctx->prof_events[ctx->prof_used].first;
-        e1 = ctx->prof_events[ctx->prof_used].second;
-        ctx->prof_used++;
-        MKV_CUDA(cudaEventRecord(e0, ctx->stream));
-    }
+    mkv_status pst = prof_begin(ctx);
+    if (pst != MKV_OK) return pst;
     if (few) {
         VerifyLaunchBatch pb;
         memset(&pb, 0, sizeof pb);
@@ -595,7 +584,7 @@ mkv_status launch_verify(Ctx *ctx, mkv_fmt fmt, VerifyItem *items_host, int n, b
         }
         for (int i = 0; i < n; i++) ctx->counter_base[i] += 2u * items_host[i].nsplit;
     }
-    if (ctx->prof) MKV_CUDA(cudaEventRecord(e1, ctx->stream));
+    if ((pst = prof_end(ctx)) != MKV_OK) return pst;
     if (any_empty && !batch && items_host[0].push != nullptr) {
         mkv_status st = launch_exchange_empty(ctx, items_host[0].push, items_host[0].push_epoch, items_host[0].ntok, items_host[0].out);
         if (st != MKV_OK) return st;

@@ -1032,6 +1032,28 @@ def test_launch_count_and_profiling(ctx, oracle):
     cache.close()
 
 
+@pytest.mark.parametrize("fmt", FMTS)
+def test_profiling_counts_prefill(ctx, fmt):
+    """Every attention core launch is timed, whichever kernels a block goes to: few tokens over a short prefix (whole items, or verify
+    items on the f32 cache), more than 64 tokens, and a block whose items are split and merged."""
+    cache = kv.KvCache(ctx, fmt, 1, 6144)
+    cache.set_len(6144)
+    q = torch.randn(500, 16, 256, device="cuda")
+    out = torch.empty_like(q)
+    ctx.prof_enable(True)
+    try:
+        for calls, (pos0, ntok) in enumerate([(100, 6), (300, 500), (5000, 40), (5000, 200)], 1):
+            cache.attn_prefill(0, 0, pos0, q[:ntok], out[:ntok])
+            ms, n = ctx.prof_read()
+            assert n == 1 and 0.0 < ms < 100.0, (pos0, ntok)
+            for _ in range(calls):
+                cache.attn_prefill(0, 0, pos0, q[:ntok], out[:ntok])
+            assert ctx.prof_read()[1] == calls
+    finally:
+        ctx.prof_enable(False)
+        cache.close()
+
+
 # ---------------------------------------------------------------- peer exchange ----------------------------------
 
 @pytest.mark.parametrize("fmt", FMTS)
