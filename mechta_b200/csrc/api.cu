@@ -1123,8 +1123,9 @@ mkv_status mkv_attn_prefill(mkv_cache *h, int layer, uint32_t first_pos, uint32_
     // than 16 of them are staged with a copy in the stream. Measured, us a layer, items / kernel: 8 tokens over 32,000 49 / 59,
     // 12 over 8,192 27 / 30, over 16,000 43 / 41; 16 over 4,096 20 / 23, over 8,192 32 / 31; 32 over 2,000 20 / 20, over 4,096
     // 31 / 25; 40 over 1,000 20 / 21, over 2,000 26 / 21; 64 over 500 20 / 20; 96 over 16 28 / 17; 300 over 4,096 466 / 89.
+    // MKV_VERIFY32=mma selects the warp-MMA kernel of the items (the measured baseline): all of the block goes there.
     const uint32_t g4 = (ntok + 3u) / 4u, g32 = (ntok + 31u) / 32u;
-    if (g4 > PARAM_ITEMS || (g4 > 2u * g32 && (uint64_t)(g4 - 2u * g32) * (end - first_pos) >= 12000u)) {
+    if (verify32_use_tc() && (g4 > PARAM_ITEMS || (g4 > 2u * g32 && (uint64_t)(g4 - 2u * g32) * (end - first_pos) >= 12000u))) {
         if ((st = prof_begin(c->ctx)) != MKV_OK) return st;
         st = launch_prefill_f32_tc(c->ctx, c, layer, first_pos, pos0, ntok, q, out);
         return st == MKV_OK ? prof_end(c->ctx) : st;

@@ -218,6 +218,8 @@ mkv_status launch_exchange_empty(Ctx *ctx, const PushInfo *push, uint32_t epoch,
 // second behind it. Both do nothing while timing is off.
 mkv_status prof_begin(Ctx *ctx);
 mkv_status prof_end(Ctx *ctx);
+// false with MKV_VERIFY32=mma: the f32 cache on the warp-MMA kernel
+bool verify32_use_tc();
 // plans the split of the items so that the grid fills the SMs once
 void plan_items(Ctx *ctx, mkv_fmt fmt, VerifyItem *items, int n);
 

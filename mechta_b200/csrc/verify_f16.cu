@@ -485,7 +485,7 @@ static bool verify_use_tc() {
 }
 // The f32 cache runs on the tcgen05 kernel of verify_f32_tc.cu; MKV_VERIFY32=mma selects the warp-MMA kernel of
 // verify_f32.cu (kept for comparison).
-static bool verify32_use_tc() {
+bool verify32_use_tc() {
     static const bool tc = [] {
         const char *e = getenv("MKV_VERIFY32");
         return !(e && strcmp(e, "mma") == 0);

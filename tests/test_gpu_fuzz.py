@@ -80,3 +80,34 @@ def test_f32_cache_on_the_warp_mma_kernel_in_a_child_process():
     r = subprocess.run([sys.executable, "-m", "pytest", os.path.join(root, "tests", "test_gpu_fuzz.py"), "-q", "-x", "-m", "gpu", "-k",
                         "random_steps"], env=env, cwd=root, capture_output=True, text=True, timeout=600)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
+
+
+def test_f32_prefill_on_the_warp_mma_kernel_in_a_child_process():
+    """MKV_VERIFY32=mma selects the warp-MMA kernel for prefill blocks of any size too: batches of 4-token items, one launch each
+    (the prefill kernel of its own takes two for a block whose items are split and merged)."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    prog = """
+import torch
+from mechta_b200 import kv
+ctx = kv.KvContext(0, torch.cuda.current_stream())
+cache = kv.KvCache(ctx, kv.KvFormat.F32, 1, 6144)
+K, V = cache.buffer_tensors(0)
+K.normal_(), V.normal_()
+cache.set_len(6144)
+for n in (40, 200):
+    q = torch.randn(n, 16, 256, device="cuda")
+    out, before = torch.empty_like(q), ctx.launches
+    cache.attn_prefill(0, 0, 5000, q, out)
+    ctx.sync()
+    assert ctx.launches - before == 1, ctx.launches - before
+    k, v = (t[:5000 + n].double().repeat_interleave(8, 1).transpose(0, 1) for t in (K, V))
+    mask = torch.ones(n, 5000 + n, dtype=torch.bool, device="cuda").tril(5000)
+    s = (q.double().transpose(0, 1) @ k.transpose(1, 2) / 16).masked_fill(~mask, float("-inf"))
+    want = (torch.softmax(s, -1) @ v).transpose(0, 1)
+    assert ((out - want).abs().max() / want.abs().max()).item() < 1e-5
+"""
+    r = subprocess.run([sys.executable, "-c", prog], env=dict(os.environ, MKV_VERIFY32="mma"), cwd=root, capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
