@@ -243,7 +243,11 @@ mkv_status mkv_attn_step(mkv_cache *c, int layer, uint32_t first_pos, uint32_t p
  * The block's K/V must already be appended (the reference appends all rows first, M/engine.rs:1213-1214).
  * q_dev [ntok][16][256]: f32 (`qr`, q_is_f16 = 0) or f16 (`qh`, the output of the reference's q_f16 pass,
  * q_is_f16 = 1; f16 cache only, as attn_fa_mx); token T sees keys first_pos <= key < pos0 + 1 + T;
- * out f32 [ntok][16][256]. 1 <= ntok <= 4096. */
+ * out f32 [ntok][16][256]. 1 <= ntok <= 4096.
+ * The partials of a block that is split over the GPU (few tokens over a long prefix) lie in 39 MB that the context takes
+ * when its first unsharded, ordinary cache is created and keeps; the call itself allocates nothing for them and can be
+ * captured. If the 39 MB are not to be had then, caches are created all the same and blocks run unsplit: the same results but
+ * for the order of sums, several times slower for few tokens over a long prefix. */
 mkv_status mkv_attn_prefill(mkv_cache *c, int layer, uint32_t first_pos, uint32_t pos0, uint32_t ntok,
                             const void *q_dev, int q_is_f16, float *out_dev);
 

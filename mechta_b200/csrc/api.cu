@@ -584,6 +584,7 @@ static mkv_status cache_create_common(mkv_ctx *h, mkv_fmt fmt, int n_layers, uin
         set_error("out of device memory for the query scratch");
         return fail(MKV_ERR_NOMEM);
     }
+    if (whole && !ring) prefill_reserve(ctx); // (prefill runs on neither shards nor rings)
     *out = reinterpret_cast<mkv_cache *>(c);
     return MKV_OK;
 }

@@ -125,7 +125,7 @@ struct Ctx {
     cudaEvent_t ev_compute = nullptr; // compute -> copy ordering
     cudaEvent_t ev_copy = nullptr;    // copy -> compute ordering
     uint32_t *dev_status = nullptr;   // device status word
-    float *pf_scratch = nullptr;      // prefill: partials of split items (prefill_tc.cu), allocated on first use
+    float *pf_scratch = nullptr;      // prefill: partials of split items, two per CTA (prefill_reserve)
     uint64_t launches = 0;
     uint64_t syncs = 0;               // mkv_sync calls so far: what was enqueued before the last of them has finished
     bool pdl = true; // programmatic dependent launch of the attention kernels (MKV_PDL=0 switches it off)
@@ -220,6 +220,10 @@ mkv_status prof_begin(Ctx *ctx);
 mkv_status prof_end(Ctx *ctx);
 // false with MKV_VERIFY32=mma: the f32 cache on the warp-MMA kernel
 bool verify32_use_tc();
+// The context's scratch for the partials of split prefill items (39 MB), taken with the first cache that prefill runs on: a launch's
+// plan, and with it the order of its sums, then depends on the call alone, also when the context's first prefill is being captured.
+// Where the memory is not there the context does without for this cache (whole items) and the next cache tries again.
+void prefill_reserve(Ctx *ctx);
 // plans the split of the items so that the grid fills the SMs once
 void plan_items(Ctx *ctx, mkv_fmt fmt, VerifyItem *items, int n);
 

@@ -85,9 +85,7 @@ __host__ __device__ inline size_t pf_slot(uint32_t pair, uint32_t piece, uint32_
 struct PfCost {
     float segment, merge, part;
 };
-// The plan of a launch, with the context's scratch of two partials per CTA in place if the plan needs it. The scratch is allocated
-// for the context's first launch that splits items and kept until the context goes; where it cannot be had (no memory left, or the
-// stream is being captured) items stay whole.
+// The plan of a launch. Without the partials' scratch (prefill_reserve) items stay whole.
 PfPlan pf_plan(Ctx *ctx, const PfCost &cost, uint32_t first_pos, uint32_t pos0, uint32_t ntok);
 // Merges the split items of the launch in front, if it has any.
 mkv_status launch_prefill_merge(Ctx *ctx, const PfPlan &plan, float *out);

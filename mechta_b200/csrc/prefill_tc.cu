@@ -650,15 +650,12 @@ static bool pf_splits(const PfPlan &plan) {
     return false;
 }
 
-static bool pf_scratch(Ctx *ctx) {
-    if (ctx->pf_scratch) return true;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(ctx->stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone &&
-        cudaMalloc(&ctx->pf_scratch, 2u * (size_t)ctx->sm_count * PF_PART * sizeof(float)) == cudaSuccess)
-        return true;
-    cudaGetLastError();
-    ctx->pf_scratch = nullptr;
-    return false;
+void prefill_reserve(Ctx *ctx) {
+    if (ctx->pf_scratch) return;
+    if (cudaMalloc(&ctx->pf_scratch, 2u * (size_t)ctx->sm_count * PF_PART * sizeof(float)) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->pf_scratch = nullptr;
+    }
 }
 
 // Chooses the way of the three that the cost model expects to be the fastest. Whole items need no merge but leave pairs idle
@@ -706,7 +703,7 @@ PfPlan pf_plan(Ctx *ctx, const PfCost &cost, uint32_t first_pos, uint32_t pos0, 
             plan.pairs = per * n;
         }
     }
-    if (pf_splits(plan) && !pf_scratch(ctx)) {
+    if (!ctx->pf_scratch && pf_splits(plan)) {
         plan.per = 1;
         plan.pairs = std::min(n, npairs);
     }

@@ -820,8 +820,8 @@ def test_prefill_f32_tile_and_split_edges(ctx, oracle, prefix, ntok, first):
 
 @pytest.mark.parametrize("fmt", FMTS)
 def test_first_prefill_of_a_context_under_capture(fmt):
-    """A launch that would split its items, captured before the context has the scratch for it, keeps them whole; the graph's result
-    is that of the split launch but for the order of sums."""
+    """A context's first prefill, recorded under capture, is planned as any later one: the scratch for split items comes with the cache,
+    so the graph's result and the later call's have the same bits (5,000 keys for 40 tokens are split)."""
     stream = torch.cuda.Stream()
     with torch.cuda.stream(stream):
         own = kv.KvContext(0, stream)
@@ -838,7 +838,7 @@ def test_first_prefill_of_a_context_under_capture(fmt):
         graph.replay()
         cache.attn_prefill(0, 0, 5000, q, want)
         own.sync()
-    assert ((out - want).norm() / want.norm()).item() < (1e-3 if fmt == kv.KvFormat.F16 else 2e-6)
+    assert torch.isfinite(want).all() and torch.equal(out, want)
     del graph
     cache.close()
     own.close()
