@@ -445,9 +445,7 @@ __device__ __forceinline__ void finish_item(const VerifyItem &it, FinishSmem &sm
         } else {
             for (uint32_t j = first + R * w; j < jobs; j += R * (NT / 32u)) merge_row_warp<NT, EXT, 2>(it, j & 1u, j >> 1, 0u);
         }
-        return;
-    }
-    if (!it.partial) { // one row a CTA at most
+    } else if (!it.partial) { // one row a CTA at most
         const uint32_t kvh = few ? first & 1u : first >> 5, row = few ? first >> 1 : first & 31u;
         if (first < jobs && row < 8u * it.ntok) merge_row_cta<NT, EXT>(it, kvh, row, sm);
     } else {
