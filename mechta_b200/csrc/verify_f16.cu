@@ -678,7 +678,8 @@ extern "C" mkv_status mkv_attn_verify_static(int device, void *stream, const voi
     if (st != MKV_OK) return st;
     const StaticDevice &d = g_static_dev[device];
 
-    // the same plan as mkv_attn_verify: contiguous runs of 64-key tiles, one CTA per SM at most
+    // contiguous runs of this kernel's 64-key tiles, one CTA per SM at most (mkv_attn_verify's pieces are whole 128-key tiles, those of
+    // its kernel: plan_items)
     VerifyLaunch L;
     memset(&L, 0, sizeof L);
     VerifyItem &it = L.item;
@@ -782,9 +783,13 @@ namespace mkv {
 //
 // The pieces of a single item are whole numbers of the kernels' 128-key tiles (`step` units). A tile costs the same MMAs and
 // softmax whether it is full or not, and a short context's first tile is loaded while the kernel in front still runs, so
-// smaller pieces only make more CTAs to wait for and more pieces to merge. us a layer in a chain, 4 tokens, f16, pieces of
-// any number of 64-key units / of whole tiles: 1,000 tokens 12.9 / 10.9, 4,096 12.6 / 11.9, 14,000 15.2 / 14.0, 23,451 17.5 /
-// 16.3, 40,000 21.9 / 21.5, the same at 65,536; f32 (32-key units): 500 18.9 / 16.8, 14,000 24.6 / 23.9, 40,000 45.0 / 44.3.
+// smaller pieces only make more CTAs to wait for and more pieces to merge. us a layer in a chain, 4 tokens, pieces of any number of
+// units (64 keys f16, 32 keys f32) / of whole tiles: f16 500 tokens 10.0 / 10.0, 1,000 10.1 / 9.9, 4,096 11.3 / 10.4, 14,000 13.7 /
+// 13.0, 23,451 15.9 / 15.1, 40,000 20.5 / 20.5, 66,400 29.5 / 28.7, 70,000 30.4 / 29.8, 110,000 41.2 / 41.2; f32 500 16.2 / 15.9,
+// 4,096 18.7 / 17.3, 14,000 24.4 / 23.5, 40,000 44.5 / 43.8, 70,000 64.9 / 63.5. (At 9,001 and 65,536 both have the same pieces.)
+// What it costs is a little of the accidental exactness of short pieces (the key with a piece's highest score has weight 1, which no
+// format rounds): error against 64 bits, 2-norm, f16 1,000 tokens 2.61e-4 / 2.71e-4, 4,096 2.64e-4 / 2.70e-4, f32 500 0.94e-6 /
+// 1.01e-6, 4,096 1.02e-6 / 1.08e-6, against 2.7e-4 to 2.9e-4 and 1.05e-6 to 1.14e-6 from 9,001 on either way.
 // A batch shares one piece length among its items, and the finer step comes closer to one wave (25 sessions of 1,701 to 4,700
 // tokens: 81 us a layer, in whole tiles 98).
 void plan_items(Ctx *ctx, mkv_fmt fmt, VerifyItem *items, int n) {
