@@ -792,23 +792,26 @@ def test_prefill_tokens_do_not_feel_later_rows(ctx, fmt, prefix, ntok, row):
     assert seen >= ntok or not torch.isfinite(poisoned[seen:]).any(dim=-1).any()
 
 
-@pytest.mark.parametrize("prefix,ntok,first", [(11988, 12, 0), (11987, 12, 0), (5987, 13, 0), (12000, 33, 10000), (1968, 32, 0), (1967, 32, 0),
-                                                (936, 64, 0), (0, 65, 0), (1791, 97, 70), (383, 257, 129), (63, 448, 0), (40, 2400, 0),
-                                                (8000, 300, 7500)])
-def test_prefill_f32_tile_and_split_edges(ctx, oracle, prefix, ntok, first):
-    """The f32 prefill at the line between batched verify items and the kernel of its own (number of 4-token groups times keys), and
+@pytest.mark.parametrize("prefix,ntok,first,own", [(11988, 12, 0, True), (11987, 12, 0, False), (5987, 13, 0, True), (12000, 33, 10000, False),
+                                                    (1968, 32, 0, True), (1967, 32, 0, False), (936, 64, 0, True), (0, 65, 0, True),
+                                                    (1791, 97, 70, True), (383, 257, 129, True), (63, 448, 0, True), (40, 2400, 0, True),
+                                                    (8000, 300, 7500, True)])
+def test_prefill_f32_tile_and_split_edges(ctx, oracle, prefix, ntok, first, own):
+    """The f32 prefill on both sides of the line between batched verify items and the kernel of its own (number of 4-token groups times
+    keys; which side a case lies on shows in its launches: items are one, the kernel and the merge of its split items two), and
     that kernel at the edges of its key tiles (128, converted in halves of 64), token groups (32 a pair of CTAs) and of the split
     of its work (dozens of parts an item; whole items). In that kernel NaN past the block's last row does not reach the outputs."""
     fmt = kv.KvFormat.F32
     cache = kv.KvCache(ctx, fmt, 1, (prefix + ntok + 4096) // 1024 * 1024)
     kc, vc = fill_both(oracle, cache, 0, prefix + ntok, 400 + ntok)
-    # goes to the kernel of its own
-    own = ntok > 64 or ((ntok + 3) // 4 - 2 * ((ntok + 31) // 32)) * (prefix + ntok - first) >= 12000
     for t in cache.buffer_tensors(0) if own else ():
         t[prefix + ntok:] = float("nan")
     q = synth.normal(401, synth.S_Q, ntok, (ntok, 16, 256))
     out = torch.full((ntok + 1, 16, 256), float("nan"), device="cuda")
+    before = ctx.launches
     cache.attn_prefill(0, first, prefix, dev(q), out[:ntok])
+    if ntok <= 64:
+        assert ctx.launches - before == (2 if own else 1)
     ctx.sync()
     got = out.cpu().numpy()
     assert np.isnan(got[ntok]).all()  # nothing past the block is written
