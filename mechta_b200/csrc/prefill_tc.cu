@@ -12,8 +12,11 @@
 // SM traffic of the tiles (9.1 GB a layer at 2,048 tokens over a 32,768-token prefix, 8.7 TB/s with the products switched
 // off) and by the issue of products with N = 64; a pair needs half the traffic, and its products are 256x128x16 and
 // 256x256x16. Measured, ten layers of 2,048 tokens over 32,768: 12.3 -> 9.7 ms (1,170 TFLOP/s under the power cap; a few layers
-// in a burst run at 1,345). The waits use mbarrier.try_wait at its default scope: with .acquire.cluster, which costs a cache
-// invalidation each time, the same kernel took 1,032 us a layer instead of 843.
+// in a burst run at 1,345). The waits use mbarrier.try_wait and the remote arrivals mbarrier.arrive at their default scope: with
+// .acquire.cluster, which costs a cache invalidation each time, the same kernel took 1,032 us a layer instead of 843. No thread
+// loads what a thread of the other CTA stored: what crosses the pair are tiles, weights and accumulators, which TMA and the tensor
+// cores read and write (each writer's fence.proxy.async or tcgen05 fence in front of its arrival, tcgen05.commit or complete_tx
+// behind the asynchronous ones).
 //
 // Scheduling. The grid is at most one pair of CTAs per two SMs; pf_plan decides what each pair takes: whole items, equal parts
 // of items, or equal ranges of the tiles of all items laid end to end (prefill_plan.cuh). A pair walks its work segment by
@@ -578,8 +581,10 @@ prefill_merge_kernel(const __grid_constant__ PfPlan plan, const float *__restric
 // The same for items of at most PF_FEW parts (equal parts of many items, cuts of long items): a thread takes four dims of a row
 // through all parts, four loads in flight; the rows leave through shared memory as whole lines. prefill_merge_kernel's four groups
 // would be idle or half so, at 121 registers a thread: ten layers, 512 tokens over 4,096 on the f32 cache (2 parts) 1,317 ->
-// 1,248 us, 200 over 9,001 on the f16 cache (5 parts) 442 -> 428. With up to 4 items the other kernel's blocks are one wave, and
-// its four groups in parallel win (6 tokens over 849: 11.9 against 12.1 us).
+// 1,248 us, 200 over 9,001 on the f16 cache (5 parts) 442 -> 428. us a layer, this kernel never / up to 8 parts / up to 16: 512 tokens
+// over 32,768 (2 parts) 222 / 215 / 215, 200 over 9,001 41.6 / 39.4 / 39.4, 128 over 9,001 (9 parts) 30.2 / 30.2 / 29.5, 96 over 9,001
+// (12 parts) 27.0 / 27.0 / 26.6; the line at 8 leaves those last 2 % where they are. With up to 4 items both kernels' blocks are one
+// wave and it makes no difference (6 tokens over 849 14.4 and 14.5, 64 over 9,001 23.0 and 23.0).
 constexpr uint32_t PF_FEW = 8;
 __global__ void __launch_bounds__(256)
 prefill_merge_few_kernel(const __grid_constant__ PfPlan plan, const float *__restrict__ scratch, float *__restrict__ out) {

@@ -104,7 +104,9 @@ def main() -> None:
                   f"Q ready med {med('q_ready'):.2f} | first S^T med {med('st_issued0', full):.2f} | "
                   f"last O^T med {med(last, full):.2f} max {us(last, full).max():.2f} | last piece {us('piece').max():.2f} | "
                   f"exit med {med('exit'):.2f} max {us('exit').max():.2f}")
-            m = x[x[:, COL["ticket"]] >= len(x) - min(len(x), 64)]  # the last arrivals merge
+            rows = min(len(x), 64)  # that many arrivals merge: the last but 40, or but as many as there are (FIN_LATE)
+            first = len(x) - rows - min(len(x) - rows, 40)
+            m = x[(x[:, COL["ticket"]] >= first) & (x[:, COL["ticket"]] < first + rows)]
             if len(m):
                 print(f"  {len(m)} merging CTAs: ticket med {med('fin_ticket', m):.2f} max {us('fin_ticket', m).max():.2f} | "
                       f"all pieces published med {med('fin_seen', m):.2f} max {us('fin_seen', m).max():.2f} | "
